@@ -11,6 +11,7 @@
 #include <mutex>
 
 #include "../../include/cortado.h"
+#include "decode.cuh"
 #include "kernels.cuh"
 
 using namespace cortado;
@@ -97,7 +98,7 @@ __device__ __forceinline__ unsigned int finish_launch(Ctl& sm, const Sync& sy, b
 // Loads the float words of a chunk into a swizzled buffer (zero past nw).
 __device__ __forceinline__ void load_plain_rows(uint32_t* buf, const uint8_t* src, long long c, int nw) {
   const uint32_t* g = reinterpret_cast<const uint32_t*>(src) + c * (long long)CW;
-  for (int w = threadIdx.x; w < CW; w += NT) buf[swz(w)] = (w < nw) ? g[w] : 0u;
+  for (int w = threadIdx.x; w < CW; w += blockDim.x) buf[swz(w)] = (w < nw) ? g[w] : 0u;
 }
 
 struct StreamHdr {
@@ -763,12 +764,132 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
   flush_pending(sm, src, s ^ 1, Y, raw_word);
 }
 
+// ---- decoders' prefetch (warp FEEDER of a decoder CTA), in two parts.
+constexpr int FEEDER = TMA_TID / 32;
+
+// What resolve_stream leaves in flight until issue_stream (lane 0).
+struct Ahead {
+  unsigned long long off;  // the scanner's word
+  int csize;
+};
+
+// First part, at the start of an iteration: finds the chunk of queue index g,
+// fills its metadata slot and reads its size entry and offset word (not
+// waited for here).
+template <int OP, class Src>
+__device__ __forceinline__ void resolve_stream(Ctl& sm, int t, long long g, const Src& src, WalkState& ws, Ahead& ah) {
+  const int lane = threadIdx.x & 31;
+  StageMeta& m = sm.st[t];
+  if (g >= src.total) {
+    if (lane == 0) m.g = g;
+    return;
+  }
+  long long c;
+  const int item = src.locate(g, ws.item, c);
+  const bool fresh = item != ws.item;
+  ws.item = item;
+  if (lane == 0) {
+    const OpArgs& A = src.args(item);
+    StreamHdr h;
+    int bad;
+    if (Src::batched && !fresh) {  // the header was read for the chunk before
+      const StageMeta& o = sm.st[t ^ 1];
+      h.n = o.n;
+      h.chunks = o.chunks;
+      h.eb_e = o.eb_e;
+      bad = o.bad >= 2 ? o.bad : 0;
+    } else {
+      h = src.header(item);
+      bad = src.header_bad(item, h);
+      if (Src::batched) {
+        tensormap_acquire(src.mout(item));
+        tensormap_acquire(src.min(item));
+      }
+    }
+    m.g = g;
+    m.c = c;
+    m.item = item;
+    m.bad = bad;
+    m.n = h.n;
+    m.chunks = h.chunks;
+    m.eb_e = h.eb_e;
+    m.nw = CW;
+    if (!bad) {
+      m.nw = (int)min((long long)CW, (h.n - c * CS) / 4);
+      ah.csize = reinterpret_cast<const uint16_t*>(A.in + HDR)[c];
+      ah.off = ld_relaxed(&A.sy.offs[c]);
+      if (OP == OP_RAPPLY && m.nw == CW) prefetch_l2(A.src + c * (long long)CS, CS);
+    }
+  }
+  __syncwarp();
+}
+
+// Second part, once the payload buffer P has been read: the payload's
+// 16-byte-aligned span with one bulk copy, the ragged tail by the lanes.
+template <class Src>
+__device__ __forceinline__ void issue_stream(Ctl& sm, int t, const Src& src, uint8_t* P, const Ahead& ah) {
+  const int lane = threadIdx.x & 31;
+  StageMeta& m = sm.st[t];
+  if (m.g >= src.total || m.bad) {
+    if (lane == 0) {
+      m.csize = 0;
+      m.d = 0;
+      m.tma_len = 0;
+      mbar_arrive(&sm.bar[0]);
+      mbar_arrive(&sm.bar[0]);
+    }
+    return;
+  }
+  const OpArgs& A = src.args(m.item);
+  unsigned long long off = 0;
+  if (lane == 0)
+    off = ((ah.off >> 48) == sm.epoch && (ah.off & LB_INC)) ? ah.off & LB_VAL : wait_offset(A.sy, sm.epoch, m.c);
+  off = __shfl_sync(0xffffffffu, off, 0);
+  const int cs = __shfl_sync(0xffffffffu, ah.csize, 0);
+  const int osize = 4 * m.nw;
+  const uint8_t* data = A.in + HDR + 2 * m.chunks;
+  const long long data_bytes = A.in_bytes - HDR - 2 * m.chunks;
+  const int bad = (cs > osize) || (cs < 2 && cs != osize) || ((long long)off + cs > data_bytes);
+  const uintptr_t Aa = reinterpret_cast<uintptr_t>(data + off);
+  const uintptr_t a0 = Aa & ~uintptr_t(15);
+  uintptr_t a1 = (Aa + (bad ? 0 : cs)) & ~uintptr_t(15);
+  if (a1 < a0) a1 = a0;
+  // The copy may run into the next payload's bytes: it takes the ragged tail
+  // too unless that would read past the stream's valid bytes.
+  const uintptr_t a1_up = (Aa + (bad ? 0 : cs) + 15) & ~uintptr_t(15);
+  if (!bad && a1_up <= reinterpret_cast<uintptr_t>(A.in + A.in_bytes)) a1 = a1_up;
+  const int d = (int)(Aa - a0);
+  const int tma_len = (int)(a1 - a0);
+  if (lane == 0) {
+    fence_proxy_async();
+    if (tma_len) {
+      mbar_expect_tx(&sm.bar[0], (uint32_t)tma_len);
+      bulk_load(P, reinterpret_cast<const void*>(a0), (uint32_t)tma_len, &sm.bar[0]);
+    } else {
+      mbar_arrive(&sm.bar[0]);
+    }
+    m.bad = bad;
+    m.csize = bad ? 0 : cs;
+    m.d = d;
+    m.tma_len = tma_len;
+  }
+  if (!bad) {
+    const uint8_t* gsrc = data + off;
+    const int from = tma_len - d;  // payload bytes [from, cs) are copied by the lanes
+    for (int i = lane + (from > 0 ? from : 0); i < cs; i += 32) P[d + i] = gsrc[i];
+  }
+  __syncwarp();
+  if (lane == 0) mbar_arrive(&sm.bar[0]);
+}
+
 // storage decode / init_recv / resi_recv (d_server_decode_kernel,
-// d_client_decode_kernel, d_residual_apply_kernel).  The payload is expanded
-// in place in its stage buffer, which then stages the output floats for one
-// TMA store.  resi_recv's client chunk is loaded behind the next payload in
-// the other stage buffer when that payload is small, else into this stage's
-// buffer after the decode.
+// d_client_decode_kernel, d_residual_apply_kernel).  Buffer 0 (P) holds the
+// payload, buffer 1 (Q) the BIT_4 planes and then the output floats for one
+// TMA store.  The next payload is loaded into P as soon as this one has been
+// expanded, while the planes are turned back into floats; its size and offset
+// are read at the start of the iteration.  resi_recv's client chunk is loaded
+// behind the next payload when that is small, else into Q once the planes
+// have been read.
 template <int OP, class Src>
 __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync& sy) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -776,104 +897,103 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
   __syncthreads();
   if (gridDim.x == 1 && warp == 1) src.scan(sm.epoch);
   __syncthreads();
+  uint32_t* P = stage_buf(sm, 0);
+  uint32_t* Q = stage_buf(sm, 1);
+  const bool feeder = warp == FEEDER;
   WalkState ws{-1};
+  Ahead ah{0, 0};
   long long pending = 0;
-  if (warp == 3) {
+  if (feeder) {
     long long g0 = 0;
     if (lane == 0) g0 = atomicAdd(&sy.counter[0], 1u);
-    g0 = __shfl_sync(0xffffffffu, g0, 0);
-    prefetch_stream(sm, 0, g0, src, ws);
+    resolve_stream<OP>(sm, 0, __shfl_sync(0xffffffffu, g0, 0), src, ws, ah);
     if (lane == 0) pending = atomicAdd(&sy.counter[0], 1u);
+    issue_stream(sm, 0, src, reinterpret_cast<uint8_t*>(P), ah);
   }
-  __syncthreads();
-  uint32_t phase = 0;  // bits 0, 1: stages; bit 2: client chunk
+  uint32_t phase = 0;  // bit 0: payload; bit 1: client chunk
   for (int s = 0;; s ^= 1) {
+    if (!mbar_wait(&sm.bar[0], phase & 1, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
+    phase ^= 1u;
     const StageMeta& m = sm.st[s];
     if (m.g >= src.total) break;
+    if (feeder) {
+      // (every other thread is past the previous chunk's last use of this slot)
+      const long long gp = __shfl_sync(0xffffffffu, pending, 0);
+      if (lane == 0) pending = atomicAdd(&sy.counter[0], 1u);
+      resolve_stream<OP>(sm, s ^ 1, gp, src, ws, ah);
+    }
     const int item = m.item;
     const OpArgs& A = src.args(item);
     const long long c = m.c;
     const int nw = m.nw;
     const bool full = nw == CW;
-    uint32_t* P = stage_buf(sm, s);
     if (Src::batched && c == 0 && tid == 0 && m.bad < 2) *A.out_size = m.n;
-    if (!mbar_wait(&sm.bar[s], (phase >> s) & 1, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
-    phase ^= 1u << s;
-    auto next = [&]() {
-      if (warp == 3) {
-        const long long gp = __shfl_sync(0xffffffffu, pending, 0);
-        if (lane == 0) pending = atomicAdd(&sy.counter[0], 1u);
-        prefetch_stream(sm, s ^ 1, gp, src, ws);
-        if (OP == OP_RAPPLY && lane == 0) {
-          // When the next payload fills at most the first KiB of the other
-          // stage buffer, this chunk's client floats are loaded behind it
-          // (1024-byte aligned) now, overlapping the decode, instead of into
-          // this stage's buffer once the decode has read it back.  A next
-          // chunk that is present and usable means prefetch_stream has waited
-          // for that buffer's previous TMA store and fenced the proxies.
-          const StageMeta& mn = sm.st[s ^ 1];
-          const bool side = full && A.has_map_in && m.bad == 0 && mn.g < src.total && mn.bad == 0 &&
-                            mn.tma_len <= 1024 && mn.d + mn.csize <= 1024;
-          sm.src_side = side ? 1u : 0u;
-          if (side) {
-            mbar_expect_tx(&sm.bar_src, CS);
-            tma_load_rows(stage_buf(sm, s ^ 1) + 256, src.min(item), (int)(c * 128), &sm.bar_src);
-          }
+    auto q_free = [&]() {
+      if (tid == TMA_TID) bulk_wait_read();  // the previous chunk's TMA store has read Q
+    };
+    const ChunkKind kind = full ? rze_decode<true>(sm, A.sy, m, P, Q, q_free) : decode_partial(sm, A.sy, m, P, Q, q_free);
+    if (feeder) {
+      issue_stream(sm, s ^ 1, src, reinterpret_cast<uint8_t*>(P), ah);
+      if (OP == OP_RAPPLY && lane == 0) {
+        // When the next payload fills at most the first KiB of P, this chunk's
+        // client floats are loaded behind it (1024-byte aligned) now.
+        const StageMeta& mn = sm.st[s ^ 1];
+        const bool side = full && A.has_map_in && m.bad == 0 && mn.g < src.total && mn.bad == 0 &&
+                          mn.tma_len <= 1024 && mn.d + mn.csize <= 1024;
+        sm.src_side = side ? 1u : 0u;
+        if (side) {
+          mbar_expect_tx(&sm.bar_src, CS);
+          tma_load_rows(P + 256, src.min(item), (int)(c * 128), &sm.bar_src);
         }
       }
-    };
-    uint32_t v[32];
-    bool raw;
-    if (full) {
-      decode_core<true>(sm, A.sy, m, P, P, v, raw, next);
-    } else {
-      next();
-      raw = decode_core_partial(sm, A.sy, m, P, P, NoHook{});
-      row_load(P, tid, v);
     }
-    if (m.bad >= 2) {  // unusable stream header (batched): nothing to write
-      __syncthreads();
-      continue;
+    if (m.bad >= 2) continue;  // unusable stream header (batched): nothing to write
+    uint32_t v[32];
+    if (kind == CHUNK_ZERO) {
+#pragma unroll
+      for (int k = 0; k < 32; k++) v[k] = 0;
+    } else if (full && kind == CHUNK_PLANES) {
+      planes_to_words<true>(sm, Q, CW, v);
+    } else {
+      row_load(Q, tid, v);
     }
     const Quant q = make_quant(m.eb_e);
+    const FastQ fq = make_fastq(m.eb_e);
     if (OP == OP_RAPPLY) {
       // d_iRESI_4 (d_RESI_4.h:79-94): requantize the client's floats to the
-      // destination bound, add the residual, dequantize.  The client's chunk
-      // is behind the next payload (sm.src_side) or comes into this stage's
-      // buffer once the decoder has read it back.
-      __syncthreads();  // sm.src_side
-      const bool src_tma = full && A.has_map_in;
-      const uint32_t* S = P;  // where the client's chunk is
-      if (src_tma) {
+      // destination bound, add the residual, dequantize.
+      if (!full || kind != CHUNK_PLANES) __syncthreads();  // sm.src_side; Q has been read
+      const uint32_t* S = Q;  // where the client's chunk is
+      if (full && A.has_map_in) {
         if (sm.src_side) {
-          S = stage_buf(sm, s ^ 1) + 256;
+          S = P + 256;
         } else if (tid == TMA_TID) {
           fence_proxy_async();
           mbar_expect_tx(&sm.bar_src, CS);
-          tma_load_rows(P, src.min(item), (int)(c * 128), &sm.bar_src);
+          tma_load_rows(Q, src.min(item), (int)(c * 128), &sm.bar_src);
         }
-        if (!mbar_wait(&sm.bar_src, (phase >> 2) & 1, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
-        phase ^= 4u;
+        if (!mbar_wait(&sm.bar_src, (phase >> 1) & 1, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
+        phase ^= 2u;
       } else {
-        load_plain_rows(P, A.src, c, nw);
+        load_plain_rows(Q, A.src, c, nw);
         __syncthreads();
       }
-      // The client's words are read from shared memory 16 bytes at a time
-      // and folded into v in place (client bin + residual), so only one
-      // 32-word array is live.  The float forms, chosen per word in a warp
-      // that holds lossless client words or bins.
+      // The client's words are folded into v in place (client bin + residual).
+      // The float forms, chosen per word in a warp that holds lossless client
+      // words or bins.
       const uint4* Srow = reinterpret_cast<const uint4*>(S + 32 * tid);
-      const FastQ fq = make_fastq(m.eb_e);
-      uint32_t amax = 0;
+      const int x = tid & 7;
+      float amax = 0.0f;
 #pragma unroll
       for (int u = 0; u < 8; u++) {
-        const uint4 w = Srow[u ^ (tid & 7)];
-        amax = max(amax, max(max(w.x & 0x7fffffffu, w.y & 0x7fffffffu), max(w.z & 0x7fffffffu, w.w & 0x7fffffffu)));
+        const uint4 w = Srow[u ^ x];
+        amax = max3_abs(amax, __uint_as_float(w.x), __uint_as_float(w.y));
+        amax = max3_abs(amax, __uint_as_float(w.z), __uint_as_float(w.w));
       }
-      if (!__any_sync(0xffffffffu, amax >= fq.thr_bits)) {
+      if (__all_sync(0xffffffffu, amax < __uint_as_float(fq.thr_bits))) {
 #pragma unroll
         for (int u = 0; u < 8; u++) {
-          const uint4 w = Srow[u ^ (tid & 7)];
+          const uint4 w = Srow[u ^ x];
           v[4 * u] += cq_fast(w.x, fq);
           v[4 * u + 1] += cq_fast(w.y, fq);
           v[4 * u + 2] += cq_fast(w.z, fq);
@@ -882,59 +1002,47 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
       } else {
 #pragma unroll
         for (int u = 0; u < 8; u++) {
-          const uint4 w = Srow[u ^ (tid & 7)];
+          const uint4 w = Srow[u ^ x];
           v[4 * u] += cq_mixed(w.x, fq, q);
           v[4 * u + 1] += cq_mixed(w.y, fq, q);
           v[4 * u + 2] += cq_mixed(w.z, fq, q);
           v[4 * u + 3] += cq_mixed(w.w, fq, q);
         }
       }
-      uint32_t bmax = 0;
+    }
+    // Chunks stored uncompressed are copied out as stored: original floats for
+    // storage decode (d_server_encode.h:234-249), request bins for init_recv
+    // (d_client_encode.h:230-254, the reference's behaviour).
+    if (OP == OP_RAPPLY || kind != CHUNK_RAW) {
+      // The float form holds for bins up to 2^23 in magnitude (that one is
+      // the lossless threshold itself in both forms).
+      float f[32], fmax = 0.0f;
 #pragma unroll
-      for (int k = 0; k < 32; k++) {
-        const uint32_t neg = (uint32_t)((int32_t)v[k] >> 31);
-        bmax = max(bmax, (v[k] ^ neg) - neg);
+      for (int k = 0; k < 32; k += 2) {
+        f[k] = __int2float_rn((int)v[k]);
+        f[k + 1] = __int2float_rn((int)v[k + 1]);
+        fmax = max3_abs(fmax, f[k], f[k + 1]);
       }
-      if (__all_sync(0xffffffffu, bmax < 0x800000u)) {
+      if (__all_sync(0xffffffffu, fmax <= 8388608.0f)) {
 #pragma unroll
-        for (int k = 0; k < 32; k++) v[k] = iq_fast(v[k], fq);
-      } else {
-#pragma unroll
-        for (int k = 0; k < 32; k++) v[k] = iq_mixed(v[k], fq, q);
-      }
-    } else if (!raw) {
-      // chunks stored uncompressed are copied out as stored: original floats
-      // for storage decode (d_server_encode.h:234-249), request bins for
-      // init_recv (d_client_encode.h:230-254, the reference's behaviour).
-      // The float dequantizer, chosen per word in a warp that holds lossless
-      // bins.
-      const FastQ fq = make_fastq(m.eb_e);
-      uint32_t bmax = 0;
-#pragma unroll
-      for (int k = 0; k < 32; k++) {
-        const uint32_t neg = (uint32_t)((int32_t)v[k] >> 31);
-        bmax = max(bmax, (v[k] ^ neg) - neg);
-      }
-      if (__all_sync(0xffffffffu, bmax < 0x800000u)) {
-#pragma unroll
-        for (int k = 0; k < 32; k++) v[k] = iq_fast(v[k], fq);
+        for (int k = 0; k < 32; k++) v[k] = __float_as_uint(__fmul_rn(f[k], fq.dsc));
       } else {
 #pragma unroll
         for (int k = 0; k < 32; k++) v[k] = iq_mixed(v[k], fq, q);
       }
     }
-    row_store(P, tid, v);  // every plane read finished before the decoder's last barrier
+    row_store(Q, tid, v);  // every plane read finished before the decoder's last barrier
     const bool tma_out = full && A.has_map_out;
     if (tma_out) fence_proxy_async();
     __syncthreads();
     if (tma_out) {
       if (tid == TMA_TID) {
-        tma_store_rows(src.mout(item), (int)(c * 128), P);
+        tma_store_rows(src.mout(item), (int)(c * 128), Q);
         bulk_commit();
       }
     } else {
       uint32_t* g = reinterpret_cast<uint32_t*>(A.out) + c * (long long)CW;
-      for (int w = tid; w < nw; w += NT) g[w] = P[swz(w)];
+      for (int w = tid; w < nw; w += NT) g[w] = Q[swz(w)];
       __syncthreads();
     }
   }

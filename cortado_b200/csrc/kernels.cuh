@@ -106,7 +106,7 @@ struct Pend {
 struct __align__(16) Ctl {
   uint16_t l2[NT];          // level-2 bitmap (2 bytes per segment thread)
   uint16_t rb[NT];          // decoder: RE1 rank base per segment thread
-  uint32_t scan_a[4], scan_b[4], scan_c[4], xchg[4];
+  uint32_t scan_a[8], scan_b[8], scan_c[8], xchg[8];
   uint64_t bar[2];          // per stage: its TMA loads
   uint64_t bar_src;         // resi_recv: the client chunk
   StageMeta st[2];
@@ -470,6 +470,7 @@ __device__ __forceinline__ void planes_to_words(Ctl& sm, const uint32_t* plane, 
   const int nw = FULL ? CW : nw_in;
   const int G = nw >> 5, rem = nw & 31;
   // ---- undo BIT_4 (d_iBIT_4): gather plane words of group g, transpose.
+  bool live = true;
   if (FULL) {
     uint32_t pe, po;
     plane_offsets(tid, pe, po);
@@ -479,7 +480,8 @@ __device__ __forceinline__ void planes_to_words(Ctl& sm, const uint32_t* plane, 
       v[s] = plane[128 * s + ((s & 1) ? po : pe)];
       any |= v[s];
     }
-    if (any) transpose32(v);
+    live = __any_sync(0xffffffffu, any != 0);  // zero planes transpose to zero words
+    if (live) transpose32(v);
   } else if (tid < G) {
 #pragma unroll
     for (int s = 0; s < 32; s++) v[s] = plane[swz(s * G + tid)];
@@ -490,11 +492,13 @@ __device__ __forceinline__ void planes_to_words(Ctl& sm, const uint32_t* plane, 
   }
   // ---- undo DIFFMS (d_iDIFFMS, d_DIFFMS.h:69-102): un-zig-zag, prefix sum.
   uint32_t acc = 0;
+  if (live) {
 #pragma unroll
-  for (int k = 0; k < 32; k++) {
-    const uint32_t z = v[k];
-    acc += (z >> 1) ^ (0u - (z & 1u));
-    v[k] = acc;
+    for (int k = 0; k < 32; k++) {
+      const uint32_t u = v[k] >> 1;
+      acc += u ^ (2u * u - v[k]);  // 2u - z is 0 or -1: z's low bit
+      v[k] = acc;
+    }
   }
   uint32_t dummy;
   const uint32_t carry = block_scan_excl(acc, sm.scan_c, dummy);  // (its barrier: every plane read is done)
