@@ -12,6 +12,7 @@
 
 #include "../../include/cortado.h"
 #include "decode.cuh"
+#include "encode.cuh"
 #include "kernels.cuh"
 
 using namespace cortado;
@@ -232,8 +233,8 @@ __device__ __forceinline__ void prefetch_floats(Ctl& sm, int t, long long g, con
   if (g >= src.total) {
     if (lane == 0) {
       m.g = g;
-      mbar_arrive(&sm.bar[t]);
-      mbar_arrive(&sm.bar[t]);
+      mbar_arrive(&sm.bar[0]);
+      mbar_arrive(&sm.bar[0]);
     }
     return;
   }
@@ -248,10 +249,10 @@ __device__ __forceinline__ void prefetch_floats(Ctl& sm, int t, long long g, con
     if (tma) {
       if (Src::batched && fresh) tensormap_acquire(src.min(item));
       fence_proxy_async();
-      mbar_expect_tx(&sm.bar[t], CS);
-      tma_load_rows(stage_buf(sm, t), src.min(item), (int)(c * 128), &sm.bar[t]);
+      mbar_expect_tx(&sm.bar[0], CS);
+      tma_load_rows(stage_buf(sm, t), src.min(item), (int)(c * 128), &sm.bar[0]);
     } else {
-      mbar_arrive(&sm.bar[t]);
+      mbar_arrive(&sm.bar[0]);
     }
     m.g = g;
     m.c = c;
@@ -261,7 +262,7 @@ __device__ __forceinline__ void prefetch_floats(Ctl& sm, int t, long long g, con
     m.n = A.n;
     m.chunks = (A.n + CS - 1) / CS;
     m.bad = 0;
-    mbar_arrive(&sm.bar[t]);
+    mbar_arrive(&sm.bar[0]);
   }
 }
 
@@ -429,86 +430,112 @@ __device__ __noinline__ void requant_words(uint32_t* buf, uint32_t m, bool raw, 
   }
 }
 
-// store (d_server_encode_kernel): floats -> SQ -> encode.  A chunk arrives in
-// buffer 0, which becomes its plane buffer; its compacted payload goes to
-// buffer 1 once the previous chunk's payload has been flushed from there (that
-// flush runs as soon as this chunk's size is published).  The next chunk is
-// loaded when the compaction has read buffer 0.
+// Resolves the pending chunk's output offset (warp 0, before a barrier that
+// publishes sm.payload_off) ...
+template <class Src>
+__device__ __forceinline__ void resolve_pending(Ctl& sm, const Src& src, const Pend& pd) {
+  if (threadIdx.x < 32 && pd.valid) {
+    const unsigned long long X = lookback_resolve(src.args(pd.item).sy, sm.epoch, pd.c, pd.csize);
+    if (threadIdx.x == 0) sm.payload_off = X;
+  }
+}
+// ... and writes it out from its staging buffer (every thread, after that
+// barrier).
+template <class Src, typename RawWord>
+__device__ __forceinline__ void write_pending(Ctl& sm, const Src& src, const Pend& pd, const uint32_t* st,
+                                              RawWord raw_word) {
+  if (!pd.valid) return;
+  const OpArgs& Q = src.args(pd.item);
+  const long long chunks = (Q.n + CS - 1) / CS;
+  const long long c = pd.c;
+  flush_staged(sm, pd, st, [&](int w) -> uint32_t { return raw_word(Q, c, w); }, Q.out + HDR + 2 * chunks,
+               reinterpret_cast<uint16_t*>(Q.out + HDR), Q.out_size, chunks);
+}
+
+// store (d_server_encode_kernel): floats -> SQ -> encode.  One buffer (A)
+// receives a chunk's floats, which are quantized into registers, and then
+// takes its planes and its payload; the other (B) holds the previous chunk's
+// payload until it is flushed, while the planes are read, and receives the next
+// chunk after that.
 template <class Src>
 __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& sy) {
+  constexpr int LOADER = 1;  // the warp that takes chunks: its planes are rarely the dense ones
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   begin_launch(sm, sy);
-  if (tid == 0) {
-    sm.pend[0].valid = 0;
-    sm.pend[1].valid = 0;
-  }
+  init_pack_table();
+  if (tid == 0) sm.pend[0].valid = sm.pend[1].valid = 0;
   WalkState ws{-1};
   __syncthreads();
-  uint32_t* A = stage_buf(sm, 0);
-  uint8_t* B = reinterpret_cast<uint8_t*>(stage_buf(sm, 1));
   // a raw chunk stores the original floats, read again from global memory
   auto raw_word = [](const OpArgs& Q, long long c, int w) -> uint32_t {
     return reinterpret_cast<const uint32_t*>(Q.in)[c * (long long)CW + w];
   };
-  auto take_next = [&]() {
-    if (warp == 3) {
-      long long g = 0;
-      if (lane == 0) g = atomicAdd(&sy.counter[0], 1u);
-      prefetch_floats(sm, 0, __shfl_sync(0xffffffffu, g, 0), src, ws);
-    }
+  auto take = [&]() -> unsigned int { return (warp == LOADER && lane == 0) ? atomicAdd(&sy.counter[0], 1u) : 0u; };
+  auto load = [&](int t, unsigned int g) {
+    if (warp == LOADER) prefetch_floats(sm, t, __shfl_sync(0xffffffffu, g, 0), src, ws);
   };
-  take_next();
-  uint32_t phase = 0;
-  int s = 0;  // pending-chunk slot of this iteration's chunk
+  load(0, take());
+  int s = 0;  // this chunk's buffer and slots; also the barrier's phase
   for (;; s ^= 1) {
-    if (!mbar_wait(&sm.bar[0], phase & 1, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
-    phase ^= 1u;
-    const StageMeta& m = sm.st[0];
+    if (!mbar_wait(&sm.bar[0], s, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
+    const StageMeta& m = sm.st[s];
     if (m.g >= src.total) break;
-    const int item = m.item;
-    const OpArgs& A_ = src.args(item);
-    const long long c = m.c;
-    const int nw = m.nw;
+    uint32_t* A = stage_buf(sm, s);
+    const OpArgs& A_ = src.args(m.item);
+    const bool full = m.nw == CW;
     if (!m.tma) {
-      load_plain_rows(A, A_.in, c, nw);
+      load_plain_rows(A, A_.in, m.c, m.nw);
       __syncthreads();
     }
-    Quant q1, q2_unused;
-    src.quant(item, q1, q2_unused);
-    if (Src::batched && c == 0 && tid == 0) write_header(A_.out, A_.n, q1.eb_e);
     uint32_t v[32];
     row_load(A, tid, v);
+    uint32_t prev0 = tid ? A[swz(32 * tid - 1)] : 0u;  // the word before (lane 0 uses it)
     {
+      Quant q1, q2_unused;
+      src.quant(m.item, q1, q2_unused);
+      if (Src::batched && tid == 0 && m.c == 0) write_header(A_.out, A_.n, q1.eb_e);
       // the float form; a warp that holds lossless words (inf, NaN included)
       // chooses per word
       const FastQ fq = make_fastq(q1.eb_e);
-      uint32_t amax = 0;
+      float amax = fabsf(__uint_as_float(prev0));
 #pragma unroll
-      for (int k = 0; k < 32; k++) amax = max(amax, v[k] & 0x7fffffffu);
-      if (!__any_sync(0xffffffffu, amax >= fq.thr_bits)) {
+      for (int k = 0; k < 32; k += 2) amax = max3_abs(amax, __uint_as_float(v[k]), __uint_as_float(v[k + 1]));
+      if (__all_sync(0xffffffffu, amax < __uint_as_float(fq.thr_bits))) {
 #pragma unroll
         for (int k = 0; k < 32; k++) v[k] = sq_fast(v[k], fq);
+        prev0 = sq_fast(prev0, fq);
       } else {
 #pragma unroll
         for (int k = 0; k < 32; k++) v[k] = sq_mixed(v[k], fq, q1);
+        prev0 = sq_mixed(prev0, fq, q1);
       }
     }
-    auto flush_prev = [&]() {
-      flush_pending(sm, src, s ^ 1, B, raw_word);
-      __syncthreads();  // buffer 1 has been read
-    };
-    if (nw == CW) {
-      encode_stage<true>(sm, A_.sy, v, A, B, c, nw, item, sm.pend[s], flush_prev);
+    __syncthreads();  // A has been read; the pending payload is complete
+    if (full) {
+      unsigned int g = 0;
+      Packer pz(0), pk(0);
+      encode_chunk<true>(
+          sm, A_.sy, v, prev0, A, m, sm.pend[s], pz, pk, [&]() { resolve_pending(sm, src, sm.pend[s ^ 1]); },
+          [&]() {
+            g = take();
+            write_pending(sm, src, sm.pend[s ^ 1], stage_buf(sm, s ^ 1), raw_word);
+          },
+          [&]() { load(s ^ 1, g); });
+      __syncthreads();  // the payload's full words are in place
+      pz.finish(A);
+      pk.finish(A);
     } else {
-      flush_prev();
       row_store(A, tid, v);
-      encode_stage_partial(sm, A_.sy, A, B, c, nw, item, sm.pend[s]);
+      resolve_pending(sm, src, sm.pend[s ^ 1]);
+      __syncthreads();
+      write_pending(sm, src, sm.pend[s ^ 1], stage_buf(sm, s ^ 1), raw_word);
+      encode_partial(sm, A_.sy, prev0, A, m, sm.pend[s]);
+      load(s ^ 1, take());
     }
-    if (tid == 0) sm.pend[s ^ 1].valid = 0;
-    __syncthreads();  // buffer 0 has been read
-    take_next();
   }
-  flush_pending(sm, src, s ^ 1, B, raw_word);
+  resolve_pending(sm, src, sm.pend[s ^ 1]);
+  __syncthreads();
+  write_pending(sm, src, sm.pend[s ^ 1], stage_buf(sm, s ^ 1), raw_word);
 }
 
 // The client side of a served request, fused into init_send / resi_send

@@ -273,25 +273,21 @@ __device__ __forceinline__ uint32_t bit_select(uint32_t x, uint32_t y, uint32_t 
   asm("lop3.b32 %0, %1, %2, %3, 0xd8;" : "=r"(r) : "r"(x), "r"(y), "r"(m));
   return r;
 }
-template <int J>
-__device__ __forceinline__ void swap_stage(uint32_t (&a)[32], uint32_t m) {
+template <int J, int N>
+__device__ __forceinline__ void swap_stage(uint32_t (&a)[N], uint32_t m) {
 #pragma unroll
-  for (int i = 0; i < 16; i++) {
+  for (int i = 0; i < N / 2; i++) {
     const int k = (i / J) * 2 * J + (i % J);
     const uint32_t x = a[k], y = a[k + J];
     a[k] = bit_select(x, y >> J, m);
     a[k + J] = bit_select(x << J, y, m);
   }
 }
-__device__ __forceinline__ void transpose32(uint32_t (&a)[32]) {
+// The stages below 16: N rows, in blocks of 16.
+template <int N>
+__device__ __forceinline__ void transpose_blocks(uint32_t (&a)[N]) {
 #pragma unroll
-  for (int k = 0; k < 16; k++) {
-    const uint32_t x = a[k], y = a[k + 16];
-    a[k] = __byte_perm(x, y, 0x3276);
-    a[k + 16] = __byte_perm(x, y, 0x1054);
-  }
-#pragma unroll
-  for (int i = 0; i < 16; i++) {
+  for (int i = 0; i < N / 2; i++) {
     const int k = (i / 8) * 16 + (i % 8);
     const uint32_t x = a[k], y = a[k + 8];
     a[k] = __byte_perm(x, y, 0x3715);
@@ -301,12 +297,50 @@ __device__ __forceinline__ void transpose32(uint32_t (&a)[32]) {
   swap_stage<2>(a, 0x33333333u);
   swap_stage<1>(a, 0x55555555u);
 }
+__device__ __forceinline__ void transpose32(uint32_t (&a)[32]) {
+#pragma unroll
+  for (int k = 0; k < 16; k++) {
+    const uint32_t x = a[k], y = a[k + 16];
+    a[k] = __byte_perm(x, y, 0x3276);
+    a[k + 16] = __byte_perm(x, y, 0x1054);
+  }
+  transpose_blocks(a);
+}
+// The same for 32 words below 2^16 (planes 0..15 are zero): words k and k + 16
+// share a register, so the stages run on 16 registers, which end up as planes
+// 16..31; and back.  128 and 112 instructions fewer than transpose32.
+__device__ __forceinline__ void narrow_to_planes(const uint32_t (&a)[32], uint32_t (&p)[16]) {
+#pragma unroll
+  for (int k = 0; k < 16; k++) p[k] = __byte_perm(a[k], a[k + 16], 0x1054);
+  transpose_blocks(p);
+}
+__device__ __forceinline__ void planes_to_narrow(uint32_t (&p)[16], uint32_t (&a)[32]) {
+  transpose_blocks(p);
+#pragma unroll
+  for (int k = 0; k < 16; k++) {
+    a[k] = p[k] >> 16;
+    a[k + 16] = p[k] & 0xffffu;
+  }
+}
 
 // ---------------------------------------------------------------- byte masks
 // 4-bit mask of the non-zero bytes of x (bit b <-> byte b).
 __device__ __forceinline__ uint32_t nz_nibble(uint32_t x) {
   const uint32_t h = (((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x) & 0x80808080u;
   return ((h >> 7) * 0x01020408u) >> 24;
+}
+// 32-bit mask of the non-zero bytes of eight words (bit 4i + b <-> byte b of
+// word i).  A four-way byte dot product with weights 1, 2, 4, 8 (16, .., 128 for
+// the second word) gathers a pair's flags, 128 each, in one accumulator.
+__device__ __forceinline__ uint32_t nz_bytes8(const uint32_t* x) {
+  uint32_t s[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const uint32_t h0 = (((x[2 * i] & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x[2 * i]) & 0x80808080u;
+    const uint32_t h1 = (((x[2 * i + 1] & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x[2 * i + 1]) & 0x80808080u;
+    s[i] = __dp4a(h0, 0x08040201u, __dp4a(h1, 0x80402010u, 0u));
+  }
+  return (s[0] >> 7) + s[1] * 2u + s[2] * 512u + s[3] * 131072u;
 }
 // 8-bit mask of the non-zero nibbles of x (bit i <-> nibble i).
 __device__ __forceinline__ uint32_t nz_nibbles8(uint32_t x) {

@@ -99,7 +99,7 @@ struct Pend {
   int item;
   int nw;
   int csize;
-  int raw;
+  int raw;                  // -1: stored uncompressed (0 or 1 in the re-encoders); else the payload's word in the buffer
   int valid;
 };
 
@@ -474,14 +474,28 @@ __device__ __forceinline__ void planes_to_words(Ctl& sm, const uint32_t* plane, 
   if (FULL) {
     uint32_t pe, po;
     plane_offsets(tid, pe, po);
-    uint32_t any = 0;
+    uint32_t p[16], high = 0, any = 0;
 #pragma unroll
-    for (int s = 0; s < 32; s++) {
+    for (int s = 0; s < 16; s++) {
       v[s] = plane[128 * s + ((s & 1) ? po : pe)];
-      any |= v[s];
+      high |= v[s];
     }
-    live = __any_sync(0xffffffffu, any != 0);  // zero planes transpose to zero words
-    if (live) transpose32(v);
+#pragma unroll
+    for (int s = 0; s < 16; s++) {
+      p[s] = plane[128 * (16 + s) + ((s & 1) ? po : pe)];
+      any |= p[s];
+    }
+    if (__any_sync(0xffffffffu, high != 0)) {
+#pragma unroll
+      for (int s = 0; s < 16; s++) v[16 + s] = p[s];
+      transpose32(v);
+    } else {
+      live = __any_sync(0xffffffffu, any != 0);  // zero planes transpose to zero words
+      if (live) planes_to_narrow(p, v);
+      else
+#pragma unroll
+        for (int s = 0; s < 16; s++) v[16 + s] = 0;
+    }
   } else if (tid < G) {
 #pragma unroll
     for (int s = 0; s < 32; s++) v[s] = plane[swz(s * G + tid)];
