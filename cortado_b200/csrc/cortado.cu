@@ -57,8 +57,7 @@ constexpr int TMA_TID = 96;
 __device__ __forceinline__ void begin_launch(Ctl& sm, const Sync& sy) {
   if (threadIdx.x == 0) sm.epoch = *(volatile unsigned int*)sy.epoch;
   if (threadIdx.x == TMA_TID) {
-    mbar_init(&sm.bar[0], 2);
-    mbar_init(&sm.bar[1], 2);
+    mbar_init(&sm.bar, 2);
     mbar_init(&sm.bar_src, 1);
     fence_mbar_init();
   }
@@ -233,8 +232,8 @@ __device__ __forceinline__ void prefetch_floats(Ctl& sm, int t, long long g, con
   if (g >= src.total) {
     if (lane == 0) {
       m.g = g;
-      mbar_arrive(&sm.bar[0]);
-      mbar_arrive(&sm.bar[0]);
+      mbar_arrive(&sm.bar);
+      mbar_arrive(&sm.bar);
     }
     return;
   }
@@ -249,10 +248,10 @@ __device__ __forceinline__ void prefetch_floats(Ctl& sm, int t, long long g, con
     if (tma) {
       if (Src::batched && fresh) tensormap_acquire(src.min(item));
       fence_proxy_async();
-      mbar_expect_tx(&sm.bar[0], CS);
-      tma_load_rows(stage_buf(sm, t), src.min(item), (int)(c * 128), &sm.bar[0]);
+      mbar_expect_tx(&sm.bar, CS);
+      tma_load_rows(stage_buf(sm, t), src.min(item), (int)(c * 128), &sm.bar);
     } else {
-      mbar_arrive(&sm.bar[0]);
+      mbar_arrive(&sm.bar);
     }
     m.g = g;
     m.c = c;
@@ -262,111 +261,8 @@ __device__ __forceinline__ void prefetch_floats(Ctl& sm, int t, long long g, con
     m.n = A.n;
     m.chunks = (A.n + CS - 1) / CS;
     m.bad = 0;
-    mbar_arrive(&sm.bar[0]);
+    mbar_arrive(&sm.bar);
   }
-}
-
-// Decoders: the payload offset comes from the launch's offset scanner (the
-// prefix sum of the size table that the reference's decoders form per CTA,
-// d_s2c.h:98-106).  One bulk copy brings the payload's 16-byte-aligned span;
-// the lanes copy the ragged tail.
-template <class Src>
-__device__ __forceinline__ void prefetch_stream(Ctl& sm, int t, long long g, const Src& src, WalkState& ws) {
-  const int lane = threadIdx.x & 31;
-  StageMeta& m = sm.st[t];
-  if (g >= src.total) {
-    if (lane == 0) {
-      m.g = g;
-      mbar_arrive(&sm.bar[t]);
-      mbar_arrive(&sm.bar[t]);
-    }
-    return;
-  }
-  long long c;
-  const int item = src.locate(g, ws.item, c);
-  const bool fresh = item != ws.item;
-  ws.item = item;
-  const OpArgs& A = src.args(item);
-  const StreamHdr h = src.header(item);
-  const int hb = src.header_bad(item, h);
-  if (hb) {
-    if (lane == 0) {
-      m.g = g;
-      m.c = c;
-      m.item = item;
-      m.nw = CW;
-      m.tma = 0;
-      m.bad = hb;
-      m.csize = 0;
-      m.d = 0;
-      m.n = 0;
-      m.chunks = 0;
-      m.eb_e = 1;
-      mbar_arrive(&sm.bar[t]);
-      mbar_arrive(&sm.bar[t]);
-    }
-    return;
-  }
-  const long long chunks = h.chunks;
-  const int nw = (int)min((long long)CW, (h.n - c * CS) / 4);
-  const int osize = nw * 4;
-  const uint16_t* table = reinterpret_cast<const uint16_t*>(A.in + HDR);
-  const uint8_t* data = A.in + HDR + 2 * chunks;
-  const long long data_bytes = A.in_bytes - HDR - 2 * chunks;
-  unsigned long long off = 0;
-  int cs = 0;
-  if (lane == 0) {
-    cs = table[c];  // in flight together with the offset read
-    off = wait_offset(A.sy, sm.epoch, c);
-  }
-  off = __shfl_sync(0xffffffffu, off, 0);
-  cs = __shfl_sync(0xffffffffu, cs, 0);
-  const int bad = (cs > osize) || (cs < 2 && cs != osize) || ((long long)off + cs > data_bytes);
-  const uintptr_t Aa = reinterpret_cast<uintptr_t>(data + off);
-  const uintptr_t a0 = Aa & ~uintptr_t(15);
-  uintptr_t a1 = (Aa + (bad ? 0 : cs)) & ~uintptr_t(15);
-  if (a1 < a0) a1 = a0;
-  // The copy may run into the next payload's bytes: it takes the ragged tail
-  // too unless that would read past the stream's valid bytes.
-  const uintptr_t a1_up = (Aa + (bad ? 0 : cs) + 15) & ~uintptr_t(15);
-  if (!bad && a1_up <= reinterpret_cast<uintptr_t>(A.in + A.in_bytes)) a1 = a1_up;
-  const int d = (int)(Aa - a0);
-  const int tma_len = (int)(a1 - a0);
-  uint8_t* dst = reinterpret_cast<uint8_t*>(stage_buf(sm, t));
-  if (lane == 0) {
-    bulk_wait_read();  // a TMA store of this buffer's previous chunk may still be reading it
-    fence_proxy_async();
-    if (tma_len) {
-      if (Src::batched && fresh) tensormap_acquire(src.mout(item));
-      mbar_expect_tx(&sm.bar[t], (uint32_t)tma_len);
-      bulk_load(dst, reinterpret_cast<const void*>(a0), (uint32_t)tma_len, &sm.bar[t]);
-    } else {
-      if (Src::batched && fresh) tensormap_acquire(src.mout(item));
-      mbar_arrive(&sm.bar[t]);
-    }
-    if (Src::batched && fresh) tensormap_acquire(src.min(item));
-    m.g = g;
-    m.c = c;
-    m.item = item;
-    m.nw = nw;
-    m.tma = tma_len != 0;
-    m.bad = bad;
-    m.csize = bad ? 0 : cs;
-    m.d = d;
-    m.tma_len = tma_len;
-    m.off = off;
-    m.n = h.n;
-    m.chunks = chunks;
-    m.eb_e = h.eb_e;
-  }
-  __syncwarp();
-  if (!bad) {
-    const uint8_t* gsrc = data + off;
-    const int from = tma_len - d;  // payload bytes [from, cs) are copied by the lanes
-    for (int i = lane + (from > 0 ? from : 0); i < cs; i += 32) dst[d + i] = gsrc[i];
-  }
-  __syncwarp();
-  if (lane == 0) mbar_arrive(&sm.bar[t]);
 }
 
 // ---- the three pipelined loops.  Each CTA dequeues chunk indices from the
@@ -380,30 +276,6 @@ __device__ __forceinline__ void prefetch_stream(Ctl& sm, int t, long long g, con
 // lookback word into an inclusive prefix, so no CTA waits on its
 // predecessors while it holds the SM.
 
-// Resolves and writes out the chunk pending in slot t (if any): warp 0 finds
-// its output offset, a barrier publishes it, every thread stores the payload
-// from `staging`, or a raw chunk's words from raw_word(args, chunk, w).
-// Called by every thread.
-template <class Src, typename RawWord>
-__device__ __forceinline__ void flush_pending(Ctl& sm, const Src& src, int t, const uint8_t* staging,
-                                              RawWord raw_word) {
-  Pend& pd = sm.pend[t];
-  const bool valid = pd.valid;  // written before an earlier barrier
-  if (valid && threadIdx.x < 32) {
-    const unsigned long long X = lookback_resolve(src.args(pd.item).sy, sm.epoch, pd.c, pd.csize);
-    if (threadIdx.x == 0) sm.payload_off = X;
-  }
-  __syncthreads();
-  if (valid) {
-    const OpArgs& Q = src.args(pd.item);
-    const long long chunks = (Q.n + CS - 1) / CS;
-    const long long c = pd.c;
-    flush_chunk(sm, pd, reinterpret_cast<const uint32_t*>(staging), false,
-                [&](int w) -> uint32_t { return raw_word(Q, c, w); }, Q.out + HDR + 2 * chunks,
-                reinterpret_cast<uint16_t*>(Q.out + HDR), Q.out_size, chunks);
-  }
-}
-
 // Requantization through floats (d_s2c.h:132-137, d_RESI_4.h:57-76): the
 // stored bin (or, for a raw chunk, the float itself) -> float (iSQ) -> request
 // bin (CQ), or residual = destination bin minus the request bin requantized
@@ -414,26 +286,30 @@ __device__ __forceinline__ void flush_pending(Ctl& sm, const Src& src, int t, co
 // made the loop large enough to stall on instruction fetch.  The words are
 // the calling thread's own row of a swizzled buffer (row_store before the
 // call, row_load after): a pointer to the caller's register array would put
-// that array in local memory for the whole loop.
+// that array in local memory for the whole loop.  Returns the word `before` the
+// row's first, requantized as well when `slow_before`.
 template <int OP>
-__device__ __noinline__ void requant_words(uint32_t* buf, uint32_t m, bool raw, Quant qs, Quant q1, Quant q2) {
+__device__ __noinline__ uint32_t requant_words(uint32_t* buf, uint32_t m, uint32_t before, bool slow_before, bool raw,
+                                               Quant qs, Quant q1, Quant q2) {
+  auto requant = [&](uint32_t stored) -> uint32_t {
+    const uint32_t x = raw ? stored : iq_dec(stored, qs);
+    if (OP == OP_S2C) return cq_enc(x, q1);
+    const uint32_t src_req = cq_enc(iq_dec(cq_enc(x, q1), q1), q2);
+    return cq_enc(x, q2) - src_req;
+  };
   const uint32_t base = 32u * threadIdx.x;
   for (; m; m &= m - 1) {
     const uint32_t w = swz(base + __ffs(m) - 1);
-    const uint32_t x = raw ? buf[w] : iq_dec(buf[w], qs);
-    if (OP == OP_S2C) {
-      buf[w] = cq_enc(x, q1);
-    } else {
-      const uint32_t src_req = cq_enc(iq_dec(cq_enc(x, q1), q1), q2);
-      buf[w] = cq_enc(x, q2) - src_req;
-    }
+    buf[w] = requant(buf[w]);
   }
+  return slow_before ? requant(before) : before;
 }
 
 // Resolves the pending chunk's output offset (warp 0, before a barrier that
 // publishes sm.payload_off) ...
 template <class Src>
-__device__ __forceinline__ void resolve_pending(Ctl& sm, const Src& src, const Pend& pd) {
+__device__ __forceinline__ void resolve_pending(Ctl& sm, const Src& src) {
+  const Pend& pd = sm.pend;
   if (threadIdx.x < 32 && pd.valid) {
     const unsigned long long X = lookback_resolve(src.args(pd.item).sy, sm.epoch, pd.c, pd.csize);
     if (threadIdx.x == 0) sm.payload_off = X;
@@ -442,13 +318,14 @@ __device__ __forceinline__ void resolve_pending(Ctl& sm, const Src& src, const P
 // ... and writes it out from its staging buffer (every thread, after that
 // barrier).
 template <class Src, typename RawWord>
-__device__ __forceinline__ void write_pending(Ctl& sm, const Src& src, const Pend& pd, const uint32_t* st,
+__device__ __forceinline__ void write_pending(Ctl& sm, const Src& src, const uint32_t* st, const uint32_t* st_small,
                                               RawWord raw_word) {
+  const Pend& pd = sm.pend;
   if (!pd.valid) return;
   const OpArgs& Q = src.args(pd.item);
   const long long chunks = (Q.n + CS - 1) / CS;
   const long long c = pd.c;
-  flush_staged(sm, pd, st, [&](int w) -> uint32_t { return raw_word(Q, c, w); }, Q.out + HDR + 2 * chunks,
+  flush_staged(sm, st, st_small, [&](int w) -> uint32_t { return raw_word(Q, c, w); }, Q.out + HDR + 2 * chunks,
                reinterpret_cast<uint16_t*>(Q.out + HDR), Q.out_size, chunks);
 }
 
@@ -463,7 +340,7 @@ __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   begin_launch(sm, sy);
   init_pack_table();
-  if (tid == 0) sm.pend[0].valid = sm.pend[1].valid = 0;
+  if (tid == 0) sm.pend.valid = 0;
   WalkState ws{-1};
   __syncthreads();
   // a raw chunk stores the original floats, read again from global memory
@@ -474,10 +351,11 @@ __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& 
   auto load = [&](int t, unsigned int g) {
     if (warp == LOADER) prefetch_floats(sm, t, __shfl_sync(0xffffffffu, g, 0), src, ws);
   };
+  auto flush = [&](int t) { write_pending(sm, src, stage_buf(sm, t), stage_buf(sm, t) + CW, raw_word); };
   load(0, take());
   int s = 0;  // this chunk's buffer and slots; also the barrier's phase
   for (;; s ^= 1) {
-    if (!mbar_wait(&sm.bar[0], s, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
+    if (!mbar_wait(&sm.bar, s, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
     const StageMeta& m = sm.st[s];
     if (m.g >= src.total) break;
     uint32_t* A = stage_buf(sm, s);
@@ -515,27 +393,166 @@ __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& 
       unsigned int g = 0;
       Packer pz(0), pk(0);
       encode_chunk<true>(
-          sm, A_.sy, v, prev0, A, m, sm.pend[s], pz, pk, [&]() { resolve_pending(sm, src, sm.pend[s ^ 1]); },
+          sm, A_.sy, v, prev0, A, A, A + CW, m, pz, pk, [&]() { resolve_pending(sm, src); },
           [&]() {
             g = take();
-            write_pending(sm, src, sm.pend[s ^ 1], stage_buf(sm, s ^ 1), raw_word);
+            flush(s ^ 1);
           },
-          [&]() { load(s ^ 1, g); });
+          [&](uint32_t) { load(s ^ 1, g); });
       __syncthreads();  // the payload's full words are in place
       pz.finish(A);
       pk.finish(A);
     } else {
       row_store(A, tid, v);
-      resolve_pending(sm, src, sm.pend[s ^ 1]);
+      resolve_pending(sm, src);
       __syncthreads();
-      write_pending(sm, src, sm.pend[s ^ 1], stage_buf(sm, s ^ 1), raw_word);
-      encode_partial(sm, A_.sy, prev0, A, m, sm.pend[s]);
+      flush(s ^ 1);
+      __syncthreads();
+      encode_partial(sm, A_.sy, prev0, A, A, A + CW, m);
       load(s ^ 1, take());
     }
   }
-  resolve_pending(sm, src, sm.pend[s ^ 1]);
+  resolve_pending(sm, src);
   __syncthreads();
-  write_pending(sm, src, sm.pend[s ^ 1], stage_buf(sm, s ^ 1), raw_word);
+  flush(s ^ 1);
+}
+
+// ---- stream prefetch (warp FEEDER of a decoder or re-encoder CTA), in two
+// parts.  The payload offset comes from the launch's offset scanner (the prefix
+// sum of the size table that the reference's decoders form per CTA,
+// d_s2c.h:98-106).
+constexpr int FEEDER = TMA_TID / 32;
+
+// What resolve_stream leaves in flight (lane 0), until park_stream puts it into
+// the metadata slot for issue_stream.
+struct Ahead {
+  unsigned long long off;  // the scanner's word
+  int csize;
+};
+
+// First part, at the start of an iteration: finds the chunk of queue index g,
+// fills its metadata slot and reads its size entry and offset word (not
+// waited for here).
+template <int OP, class Src>
+__device__ __forceinline__ void resolve_stream(Ctl& sm, int t, long long g, const Src& src, WalkState& ws, Ahead& ah) {
+  const int lane = threadIdx.x & 31;
+  StageMeta& m = sm.st[t];
+  ah.csize = 0;
+  if (g >= src.total) {
+    if (lane == 0) m.g = g;
+    return;
+  }
+  long long c;
+  const int item = src.locate(g, ws.item, c);
+  const bool fresh = item != ws.item;
+  ws.item = item;
+  if (lane == 0) {
+    const OpArgs& A = src.args(item);
+    StreamHdr h;
+    int bad;
+    if (Src::batched && !fresh) {  // the header was read for the chunk before
+      const StageMeta& o = sm.st[t ^ 1];
+      h.n = o.n;
+      h.chunks = o.chunks;
+      h.eb_e = o.eb_e;
+      bad = o.bad >= 2 ? o.bad : 0;
+    } else {
+      h = src.header(item);
+      bad = src.header_bad(item, h);
+      if (Src::batched) {
+        tensormap_acquire(src.mout(item));
+        tensormap_acquire(src.min(item));
+      }
+    }
+    m.g = g;
+    m.c = c;
+    m.item = item;
+    m.bad = bad;
+    m.n = h.n;
+    m.chunks = h.chunks;
+    m.eb_e = h.eb_e;
+    m.nw = CW;
+    if (!bad) {
+      m.nw = (int)min((long long)CW, (h.n - c * CS) / 4);
+      ah.csize = reinterpret_cast<const uint16_t*>(A.in + HDR)[c];
+      ah.off = ld_relaxed(&A.sy.offs[c]);
+      const uint8_t* client = OP == OP_RAPPLY ? A.src : OP == OP_RESI ? A.client : nullptr;
+      if (client && m.nw == CW) prefetch_l2(client + c * (long long)CS, CS);
+    }
+  }
+  __syncwarp();
+}
+
+template <class Src>
+__device__ __forceinline__ void park_stream(Ctl& sm, int t, const Src& src, const Ahead& ah) {
+  StageMeta& m = sm.st[t];
+  if ((threadIdx.x & 31) == 0) {
+    m.off = ah.off;
+    m.csize = ah.csize;
+  }
+  __syncwarp();
+}
+
+// Second part, once the place at byte `at` (a multiple of 16) of P is free: the
+// payload's 16-byte-aligned span with one bulk copy, the ragged tail by the
+// lanes.
+template <class Src>
+__device__ __forceinline__ void issue_stream(Ctl& sm, int t, const Src& src, uint8_t* P, int at) {
+  const int lane = threadIdx.x & 31;
+  StageMeta& m = sm.st[t];
+  if (m.g >= src.total || m.bad) {
+    if (lane == 0) {
+      m.csize = 0;
+      m.d = 0;
+      m.tma_len = 0;
+      mbar_arrive(&sm.bar);
+      mbar_arrive(&sm.bar);
+    }
+    return;
+  }
+  const OpArgs& A = src.args(m.item);
+  unsigned long long off = 0;
+  if (lane == 0) {
+    const unsigned long long w = m.off;
+    off = ((w >> 48) == sm.epoch && (w & LB_INC)) ? w & LB_VAL : wait_offset(A.sy, sm.epoch, m.c);
+  }
+  off = __shfl_sync(0xffffffffu, off, 0);
+  const int cs = m.csize;
+  __syncwarp();  // (lane 0 rewrites it below)
+  const int osize = 4 * m.nw;
+  const uint8_t* data = A.in + HDR + 2 * m.chunks;
+  const long long data_bytes = A.in_bytes - HDR - 2 * m.chunks;
+  const int bad = (cs > osize) || (cs < 2 && cs != osize) || ((long long)off + cs > data_bytes);
+  const uintptr_t Aa = reinterpret_cast<uintptr_t>(data + off);
+  const uintptr_t a0 = Aa & ~uintptr_t(15);
+  uintptr_t a1 = (Aa + (bad ? 0 : cs)) & ~uintptr_t(15);
+  if (a1 < a0) a1 = a0;
+  // The copy may run into the next payload's bytes: it takes the ragged tail
+  // too unless that would read past the stream's valid bytes.
+  const uintptr_t a1_up = (Aa + (bad ? 0 : cs) + 15) & ~uintptr_t(15);
+  if (!bad && a1_up <= reinterpret_cast<uintptr_t>(A.in + A.in_bytes)) a1 = a1_up;
+  const int d = at + (int)(Aa - a0);
+  const int tma_len = (int)(a1 - a0);
+  if (lane == 0) {
+    fence_proxy_async();
+    if (tma_len) {
+      mbar_expect_tx(&sm.bar, (uint32_t)tma_len);
+      bulk_load(P + at, reinterpret_cast<const void*>(a0), (uint32_t)tma_len, &sm.bar);
+    } else {
+      mbar_arrive(&sm.bar);
+    }
+    m.bad = bad;
+    m.csize = bad ? 0 : cs;
+    m.d = d;
+    m.tma_len = tma_len;
+  }
+  if (!bad) {
+    const uint8_t* gsrc = data + off;
+    const int from = at + tma_len - d;  // payload bytes [from, cs) are copied by the lanes
+    for (int i = lane + (from > 0 ? from : 0); i < cs; i += 32) P[d + i] = gsrc[i];
+  }
+  __syncwarp();
+  if (lane == 0) mbar_arrive(&sm.bar);
 }
 
 // The client side of a served request, fused into init_send / resi_send
@@ -652,87 +669,114 @@ __device__ __noinline__ void client_raw_bins(const OpArgs& A, long long c, int n
 // staging buffer (out of line: only chunks that do not compress take it, and
 // the re-encoders' loop is large enough to stall on instruction fetch).
 __device__ __noinline__ void raw_rebuild(Ctl& sm, const uint32_t* X, int nw, uint32_t* Yw) {
-  uint32_t w[32];
-  if (nw == CW) planes_to_words<true>(sm, X, nw, w);
-  else planes_to_words<false>(sm, X, nw, w);
+  uint32_t w[32], before;
+  if (nw == CW) planes_to_words<true>(sm, X, nw, w, before);
+  else planes_to_words<false>(sm, X, nw, w, before);
   row_store(Yw, threadIdx.x, w);
 }
 
+// Blocking flush of the re-encoders' pending chunk, outside the hot path: when
+// the next payload does not fit beside it, around partial chunks and at the end
+// of the loop.  Every earlier write to R may precede it without a barrier.
+template <class Src>
+__device__ __noinline__ void flush_now(Ctl& sm, const Src src, uint32_t* R) {
+  __syncthreads();
+  resolve_pending(sm, src);
+  __syncthreads();
+  write_pending(sm, src, R, R, [R](const OpArgs&, long long, int w) -> uint32_t { return R[swz(w)]; });
+  __syncthreads();
+  if (threadIdx.x == 0) sm.pend.valid = 0;
+}
+
 // init_send / resi_send (d_s2c_encode_kernel, d_residual_encode_kernel):
-// decode the stored chunk, requantize or form the residual, encode.  The
-// payload arrives in buffer 0 and is expanded in place; after the
-// requantization the same buffer is the encoder's plane buffer.  The compacted
-// payload goes to buffer 1 once the previous chunk has been flushed from there
-// (as in store_loop).  A chunk that does not compress stores its requantized
-// words, which are rebuilt from the plane buffer (planes_to_words) into
-// buffer 1 -- rare enough not to keep a third buffer for them.
+// decode the stored chunk, requantize or form the residual, encode.  The first
+// 16 KiB of the buffers (Y) hold the BIT_4 planes, first the stored chunk's,
+// then the new one's; in between its rows are scratch for the requantization
+// and the client's floats.  The 18 KiB behind them (R) hold the previous
+// chunk's new payload at the low end, until it is flushed while the new planes
+// are read, and the stored payload at the high end; the next one is loaded
+// there as soon as this chunk's size is known, or, when the two do not fit,
+// after a blocking flush.  A chunk that does not compress stores its
+// requantized words, which are rebuilt from the planes (planes_to_words).
+// (Decoding in place in one buffer and staging in the other took 11 barriers a
+// chunk; this takes 7.  256 MiB: init_send 462 -> 320 us and resi_send 468 ->
+// 340 us on sinusoids with noise, 552 -> 414 and 516 -> 387 us on dense data,
+// 269 -> 256 and 282 -> 277 us on nearly all zero bins.  Instruction fetch is
+// now the largest stall.)
 // APPLY: the fused send-and-apply forms (items with a client's floats); the
 // plain forms are compiled without that code.
+constexpr int ROOM = (2 * BUF_WORDS - CW) * 4;  // bytes of R
+// Bytes that a payload of n bytes takes at R's high end (any alignment, and
+// what the decoder reads past its end), and at its low end (padded).
+__device__ __forceinline__ int room_in(int n) { return ((n + 30) & ~15) + 32; }
+__device__ __forceinline__ int room_out(int n) { return n + (n >> 5) + 32; }
+
 template <int OP, bool APPLY, class Src>
 __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Sync& sy) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   begin_launch(sm, sy);
-  if (tid == 0) {
-    sm.pend[0].valid = 0;
-    sm.pend[1].valid = 0;
-  }
-  WalkState ws{-1};
+  init_pack_table();
+  if (tid == 0) sm.pend.valid = 0;
   __syncthreads();  // sm.epoch
   if (gridDim.x == 1 && warp == 1) src.scan(sm.epoch);
   __syncthreads();
-  uint32_t* X = stage_buf(sm, 0);
-  uint32_t* Yw = stage_buf(sm, 1);
-  uint8_t* Y = reinterpret_cast<uint8_t*>(Yw);
-  // a raw chunk's payload is its requantized words, kept swizzled in buffer 1
-  auto raw_word = [Yw](const OpArgs&, long long, int w) -> uint32_t { return Yw[swz(w)]; };
-  auto take_next = [&]() {
-    if (warp == 3) {
-      long long g = 0;
-      if (lane == 0) g = atomicAdd(&sy.counter[0], 1u);
-      prefetch_stream(sm, 0, __shfl_sync(0xffffffffu, g, 0), src, ws);
-      if (OP == OP_RESI && APPLY && lane == 0) {
-        // resi_send with apply reads the client's chunk: bring it into L2 now
-        const StageMeta& mn = sm.st[0];
-        if (mn.g < src.total && mn.bad == 0) {
-          const OpArgs& An = src.args(mn.item);
-          if (An.client && mn.nw == CW) prefetch_l2(An.client + mn.c * (long long)CS, CS);
-        }
-      }
-    }
+  uint32_t* Y = stage_buf(sm, 0);
+  uint32_t* R = Y + CW;
+  const bool feeder = warp == FEEDER;
+  WalkState ws{-1};
+  Ahead ah{0, 0};
+  auto take = [&]() -> unsigned int { return (feeder && lane == 0) ? atomicAdd(&sy.counter[0], 1u) : 0u; };
+  auto resolve = [&](int t, unsigned int g) {
+    if (feeder) resolve_stream<OP>(sm, t, __shfl_sync(0xffffffffu, g, 0), src, ws, ah);
   };
-  take_next();
-  uint32_t phase = 0;
-  int s = 0;  // pending-chunk slot of this iteration's chunk
-  for (;; s ^= 1) {
-    if (!mbar_wait(&sm.bar[0], phase & 1, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
-    phase ^= 1u;
-    const StageMeta& m = sm.st[0];
+  auto park = [&](int t) {
+    if (feeder) park_stream(sm, t, src, ah);
+  };
+  auto issue = [&](int t) {  // (feeder)
+    issue_stream(sm, t, src, reinterpret_cast<uint8_t*>(R), ROOM - room_in(min(sm.st[t].csize, CS)));
+  };
+  resolve(0, take());
+  park(0);
+  if (feeder) issue(0);
+  for (int s = 0;; s ^= 1) {  // s: the metadata slot, and the barrier's phase
+    if (!mbar_wait(&sm.bar, s, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
+    const StageMeta& m = sm.st[s];
     if (m.g >= src.total) break;
-    const int item = m.item;
-    const OpArgs& A = src.args(item);
-    const long long c = m.c;
-    const int nw = m.nw;
-    auto flush_prev = [&]() {
-      flush_pending(sm, src, s ^ 1, Y, raw_word);
-      __syncthreads();  // buffer 1 has been read
-    };
-    uint32_t v[32];
-    bool raw;
-    if (nw == CW) {
-      decode_core<true>(sm, A.sy, m, X, X, v, raw, NoHook{});
-    } else {
-      raw = decode_core_partial(sm, A.sy, m, X, X, NoHook{});
-      row_load(X, tid, v);
-    }
+    const OpArgs& A = src.args(m.item);
+    const bool full = m.nw == CW;
+    const ChunkKind kind =
+        full ? rze_decode<true>(sm, A.sy, m, R, Y, NoHook{}) : decode_partial(sm, A.sy, m, R, Y, NoHook{});
+    const unsigned int g = take();
     if (m.bad >= 2) {  // unusable stream header (batched): nothing to write
-      if (tid == 0) sm.pend[s].valid = 0;
-      flush_prev();
+      resolve(s ^ 1, g);
+      park(s ^ 1);
+      flush_now(sm, src, R);
+      if (feeder) issue(s ^ 1);
+      continue;
+    }
+    uint32_t v[32], before = 0;  // before: the word before this thread's first
+    if (kind == CHUNK_ZERO) {
+#pragma unroll
+      for (int k = 0; k < 32; k++) v[k] = 0;
+    } else if (full && kind == CHUNK_PLANES) {
+      planes_to_words<true>(sm, Y, CW, v, before);
     } else {
+      row_load(Y, tid, v);
+      if (!full && 32 * tid + 32 > m.nw) {
+#pragma unroll
+        for (int k = 0; k < 32; k++)
+          if (32 * tid + k >= m.nw) v[k] = 0;
+      }
+      before = (tid && 32 * tid - 1 < m.nw) ? Y[swz(32 * tid - 1)] : 0u;
+      __syncthreads();  // rows are scratch from here on
+    }
+    {
       // stored bins -> floats (iSQ, skipped for chunks stored as floats) ->
       // request bins (CQ, d_s2c.h:132-137) or residuals (d_RESI_4.h:57-76)
+      const bool raw = kind == CHUNK_RAW;
       const Quant qs = make_quant(m.eb_e);
       Quant q1, q2;
-      src.quant(item, q1, q2);
+      src.quant(m.item, q1, q2);
       // Shift form, when every word of the warp allows it: a lossy stored bin
       // a (|a| < 2^23) is the float a * 2^(e_s - 126), so its request bin is
       // a / 2^k1 rounded half away from zero (k1 = e_1 - e_s >= 0), and the
@@ -752,161 +796,69 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
                             : (OP == OP_RESI && k2 == 0 && k1 >= 1 && k1 <= 23) ? 0x800000u - (1u << (k1 - 1))
                                                                                  : 0x800000u;
       const uint32_t h1 = shl_clamp(1u, (uint32_t)(k1 - 1)), h2 = shl_clamp(1u, (uint32_t)(k2 - 1));
-      uint32_t slow = 0;
-#pragma unroll
-      for (int k = 0; k < 32; k++) {
-        const uint32_t neg = (uint32_t)((int32_t)v[k] >> 31);
-        const uint32_t a = (v[k] ^ neg) - neg;
+      auto shifted = [&](uint32_t& w) -> bool {
+        const uint32_t neg = (uint32_t)((int32_t)w >> 31);
+        const uint32_t a = (w ^ neg) - neg;
         const uint32_t m1 = shr_clamp(a + h1, (uint32_t)k1);
         const uint32_t r = (OP == OP_S2C) ? m1 : shr_clamp(a + h2, (uint32_t)k2) - shl_clamp(m1, (uint32_t)dd);
         const bool ok = a < amax;
-        slow |= (ok ? 0u : 1u) << k;
-        v[k] = ok ? (r ^ neg) - neg : v[k];
+        w = ok ? (r ^ neg) - neg : w;
+        return ok;
+      };
+      uint32_t slow = 0;
+#pragma unroll
+      for (int k = 0; k < 32; k++) slow |= (shifted(v[k]) ? 0u : 1u) << k;
+      const bool slow_before = !shifted(before);
+      if (slow | (uint32_t)slow_before) {  // row tid of Y is this thread's own
+        row_store(Y, tid, v);
+        before = requant_words<OP>(Y, slow, before, slow_before, raw, qs, q1, q2);
+        row_load(Y, tid, v);
       }
-      if (slow) {  // after the decoder's last barrier row tid of X is this thread's own
-        row_store(X, tid, v);
-        requant_words<OP>(X, slow, raw, qs, q1, q2);
-        row_load(X, tid, v);
-      }
-      if (Src::batched && c == 0 && tid == 0) write_header(A.out, m.n, (OP == OP_S2C) ? q1.eb_e : q2.eb_e);
-      if (APPLY && A.client) client_apply<OP>(A, c, nw, v, OP == OP_S2C ? q1 : q2, X);
-      if (nw == CW) {
-        encode_stage<true>(sm, A.sy, v, X, Y, c, nw, item, sm.pend[s], flush_prev);
-      } else {
-        flush_prev();
-        row_store(X, tid, v);
-        encode_stage_partial(sm, A.sy, X, Y, c, nw, item, sm.pend[s]);
-        __syncthreads();  // sm.pend[s]
-      }
-      if (sm.pend[s].raw) {
-        // the requantized words, rebuilt from the plane buffer, are the payload
-        raw_rebuild(sm, X, nw, Yw);
-        if (OP == OP_S2C && APPLY && A.client) client_raw_bins(A, c, nw, Yw);
-      }
+      if (Src::batched && m.c == 0 && tid == 0) write_header(A.out, m.n, (OP == OP_S2C) ? q1.eb_e : q2.eb_e);
+      resolve(s ^ 1, g);
+      if (APPLY && A.client) client_apply<OP>(A, m.c, m.nw, v, OP == OP_S2C ? q1 : q2, Y);
     }
-    if (tid == 0) sm.pend[s ^ 1].valid = 0;
-    __syncthreads();  // buffer 0 has been read; buffer 1 holds this chunk's payload
-    take_next();
-  }
-  flush_pending(sm, src, s ^ 1, Y, raw_word);
-}
-
-// ---- decoders' prefetch (warp FEEDER of a decoder CTA), in two parts.
-constexpr int FEEDER = TMA_TID / 32;
-
-// What resolve_stream leaves in flight until issue_stream (lane 0).
-struct Ahead {
-  unsigned long long off;  // the scanner's word
-  int csize;
-};
-
-// First part, at the start of an iteration: finds the chunk of queue index g,
-// fills its metadata slot and reads its size entry and offset word (not
-// waited for here).
-template <int OP, class Src>
-__device__ __forceinline__ void resolve_stream(Ctl& sm, int t, long long g, const Src& src, WalkState& ws, Ahead& ah) {
-  const int lane = threadIdx.x & 31;
-  StageMeta& m = sm.st[t];
-  if (g >= src.total) {
-    if (lane == 0) m.g = g;
-    return;
-  }
-  long long c;
-  const int item = src.locate(g, ws.item, c);
-  const bool fresh = item != ws.item;
-  ws.item = item;
-  if (lane == 0) {
-    const OpArgs& A = src.args(item);
-    StreamHdr h;
-    int bad;
-    if (Src::batched && !fresh) {  // the header was read for the chunk before
-      const StageMeta& o = sm.st[t ^ 1];
-      h.n = o.n;
-      h.chunks = o.chunks;
-      h.eb_e = o.eb_e;
-      bad = o.bad >= 2 ? o.bad : 0;
+    bool raw_out, held;
+    if (full) {
+      __syncthreads();  // the rows of Y are free
+      Packer pz(0), pk(0);
+      raw_out = encode_chunk<true>(
+          sm, A.sy, v, before, Y, R, R, m, pz, pk,
+          [&]() {
+            resolve_pending(sm, src);
+            park(s ^ 1);
+          },
+          [&]() {
+            write_pending(sm, src, R, R, [R](const OpArgs&, long long, int w) -> uint32_t { return R[swz(w)]; });
+          },
+          [&](uint32_t bytes) {
+            if (feeder) {
+              const int cs = min(sm.st[s ^ 1].csize, CS);
+              const bool fits = room_out(min((int)bytes, CS)) + room_in(cs) <= ROOM;
+              if (lane == 0) sm.held = !fits;
+              if (fits) issue(s ^ 1);
+            }
+          });
+      if (raw_out) raw_rebuild(sm, Y, CW, R);
+      __syncthreads();  // the payload's full words are in place
+      pz.finish(R);
+      pk.finish(R);
+      held = sm.held;
     } else {
-      h = src.header(item);
-      bad = src.header_bad(item, h);
-      if (Src::batched) {
-        tensormap_acquire(src.mout(item));
-        tensormap_acquire(src.min(item));
-      }
+      park(s ^ 1);
+      flush_now(sm, src, R);
+      row_store(Y, tid, v);
+      raw_out = encode_partial(sm, A.sy, before, Y, R, R, m);
+      if (raw_out) raw_rebuild(sm, Y, m.nw, R);
+      held = true;
     }
-    m.g = g;
-    m.c = c;
-    m.item = item;
-    m.bad = bad;
-    m.n = h.n;
-    m.chunks = h.chunks;
-    m.eb_e = h.eb_e;
-    m.nw = CW;
-    if (!bad) {
-      m.nw = (int)min((long long)CW, (h.n - c * CS) / 4);
-      ah.csize = reinterpret_cast<const uint16_t*>(A.in + HDR)[c];
-      ah.off = ld_relaxed(&A.sy.offs[c]);
-      if (OP == OP_RAPPLY && m.nw == CW) prefetch_l2(A.src + c * (long long)CS, CS);
+    if (raw_out && OP == OP_S2C && APPLY && A.client) client_raw_bins(A, m.c, m.nw, R);
+    if (held) {
+      flush_now(sm, src, R);
+      if (feeder) issue(s ^ 1);
     }
   }
-  __syncwarp();
-}
-
-// Second part, once the payload buffer P has been read: the payload's
-// 16-byte-aligned span with one bulk copy, the ragged tail by the lanes.
-template <class Src>
-__device__ __forceinline__ void issue_stream(Ctl& sm, int t, const Src& src, uint8_t* P, const Ahead& ah) {
-  const int lane = threadIdx.x & 31;
-  StageMeta& m = sm.st[t];
-  if (m.g >= src.total || m.bad) {
-    if (lane == 0) {
-      m.csize = 0;
-      m.d = 0;
-      m.tma_len = 0;
-      mbar_arrive(&sm.bar[0]);
-      mbar_arrive(&sm.bar[0]);
-    }
-    return;
-  }
-  const OpArgs& A = src.args(m.item);
-  unsigned long long off = 0;
-  if (lane == 0)
-    off = ((ah.off >> 48) == sm.epoch && (ah.off & LB_INC)) ? ah.off & LB_VAL : wait_offset(A.sy, sm.epoch, m.c);
-  off = __shfl_sync(0xffffffffu, off, 0);
-  const int cs = __shfl_sync(0xffffffffu, ah.csize, 0);
-  const int osize = 4 * m.nw;
-  const uint8_t* data = A.in + HDR + 2 * m.chunks;
-  const long long data_bytes = A.in_bytes - HDR - 2 * m.chunks;
-  const int bad = (cs > osize) || (cs < 2 && cs != osize) || ((long long)off + cs > data_bytes);
-  const uintptr_t Aa = reinterpret_cast<uintptr_t>(data + off);
-  const uintptr_t a0 = Aa & ~uintptr_t(15);
-  uintptr_t a1 = (Aa + (bad ? 0 : cs)) & ~uintptr_t(15);
-  if (a1 < a0) a1 = a0;
-  // The copy may run into the next payload's bytes: it takes the ragged tail
-  // too unless that would read past the stream's valid bytes.
-  const uintptr_t a1_up = (Aa + (bad ? 0 : cs) + 15) & ~uintptr_t(15);
-  if (!bad && a1_up <= reinterpret_cast<uintptr_t>(A.in + A.in_bytes)) a1 = a1_up;
-  const int d = (int)(Aa - a0);
-  const int tma_len = (int)(a1 - a0);
-  if (lane == 0) {
-    fence_proxy_async();
-    if (tma_len) {
-      mbar_expect_tx(&sm.bar[0], (uint32_t)tma_len);
-      bulk_load(P, reinterpret_cast<const void*>(a0), (uint32_t)tma_len, &sm.bar[0]);
-    } else {
-      mbar_arrive(&sm.bar[0]);
-    }
-    m.bad = bad;
-    m.csize = bad ? 0 : cs;
-    m.d = d;
-    m.tma_len = tma_len;
-  }
-  if (!bad) {
-    const uint8_t* gsrc = data + off;
-    const int from = tma_len - d;  // payload bytes [from, cs) are copied by the lanes
-    for (int i = lane + (from > 0 ? from : 0); i < cs; i += 32) P[d + i] = gsrc[i];
-  }
-  __syncwarp();
-  if (lane == 0) mbar_arrive(&sm.bar[0]);
+  flush_now(sm, src, R);
 }
 
 // storage decode / init_recv / resi_recv (d_server_decode_kernel,
@@ -935,11 +887,12 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     if (lane == 0) g0 = atomicAdd(&sy.counter[0], 1u);
     resolve_stream<OP>(sm, 0, __shfl_sync(0xffffffffu, g0, 0), src, ws, ah);
     if (lane == 0) pending = atomicAdd(&sy.counter[0], 1u);
-    issue_stream(sm, 0, src, reinterpret_cast<uint8_t*>(P), ah);
+    park_stream(sm, 0, src, ah);
+    issue_stream(sm, 0, src, reinterpret_cast<uint8_t*>(P), 0);
   }
   uint32_t phase = 0;  // bit 0: payload; bit 1: client chunk
   for (int s = 0;; s ^= 1) {
-    if (!mbar_wait(&sm.bar[0], phase & 1, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
+    if (!mbar_wait(&sm.bar, phase & 1, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
     phase ^= 1u;
     const StageMeta& m = sm.st[s];
     if (m.g >= src.total) break;
@@ -960,7 +913,8 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     };
     const ChunkKind kind = full ? rze_decode<true>(sm, A.sy, m, P, Q, q_free) : decode_partial(sm, A.sy, m, P, Q, q_free);
     if (feeder) {
-      issue_stream(sm, s ^ 1, src, reinterpret_cast<uint8_t*>(P), ah);
+      park_stream(sm, s ^ 1, src, ah);
+      issue_stream(sm, s ^ 1, src, reinterpret_cast<uint8_t*>(P), 0);
       if (OP == OP_RAPPLY && lane == 0) {
         // When the next payload fills at most the first KiB of P, this chunk's
         // client floats are loaded behind it (1024-byte aligned) now.
@@ -980,7 +934,8 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
 #pragma unroll
       for (int k = 0; k < 32; k++) v[k] = 0;
     } else if (full && kind == CHUNK_PLANES) {
-      planes_to_words<true>(sm, Q, CW, v);
+      uint32_t before;
+      planes_to_words<true>(sm, Q, CW, v, before);
     } else {
       row_load(Q, tid, v);
     }

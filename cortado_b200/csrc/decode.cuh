@@ -240,7 +240,8 @@ __device__ __noinline__ ChunkKind decode_partial(Ctl& sm, const Sync& sy, const 
   const ChunkKind kind = rze_decode<false>(sm, sy, m, P, Q, q_free);
   if (kind != CHUNK_PLANES) return kind;
   uint32_t w[32];
-  planes_to_words<false>(sm, Q, m.nw, w);
+  uint32_t before;
+  planes_to_words<false>(sm, Q, m.nw, w, before);
   row_store(Q, threadIdx.x, w);
   return kind;
 }

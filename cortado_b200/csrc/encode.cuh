@@ -87,19 +87,21 @@ struct Packer {
 // Input: v[32] = the pre-DIFFMS words of group g = threadIdx.x (quantized bins
 // or residuals; words at or beyond nw are 0) and, for lane 0, the word before
 // them (prev0, 0 for thread 0).  Y is free on entry; it becomes the plane
-// buffer (d_DIFFMS_4 -> d_BIT_4 -> d_RZE_1, raw fallback) and then holds the
-// payload, padded (staged()), until flush_chunk writes it out.  The chunk's
-// size is published for the lookback and the chunk recorded in `pend`.  A raw
-// chunk leaves the planes in Y.  A payload of at most SMALL bytes is staged
-// behind the planes instead.  The caller holds a barrier after this, then every
+// buffer (d_DIFFMS_4 -> d_BIT_4 -> d_RZE_1, raw fallback).  The payload goes,
+// padded (staged()), to `st`, which may be Y itself and is not written before
+// the planes have been read, or unpadded to `st_small` (not Y) when it has at
+// most SMALL bytes, and stays there until flush_staged writes it out.  The
+// chunk's size is published for the lookback and the chunk recorded in sm.pend.
+// Returns whether the chunk is stored raw; then nothing is staged and the
+// planes are still in Y.  The caller holds a barrier after this, then every
 // thread finishes its runs pz and pk.
 // Three hooks run on every thread: planes_written() before the barrier after
-// which the planes are read, planes_ready() after it and planes_read() after
-// the next one.
+// which the planes are read, planes_ready() after it, and planes_read(n) after
+// the next one, with a bound n of the payload's bytes.
 // FULL: a whole 16 KiB chunk (nw == 4096), with compile-time addressing.
 template <bool FULL, typename Written, typename Ready, typename Read>
-__device__ __forceinline__ void encode_chunk(Ctl& sm, const Sync& sy, uint32_t (&v)[32], uint32_t prev0, uint32_t* Y,
-                                             const StageMeta& m, Pend& pend, Packer& pz, Packer& pk,
+__device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (&v)[32], uint32_t prev0, uint32_t* Y,
+                                             uint32_t* st, uint32_t* st_small, const StageMeta& m, Packer& pz, Packer& pk,
                                              Written planes_written, Ready planes_ready, Read planes_read) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nw = FULL ? CW : m.nw;
@@ -155,14 +157,13 @@ __device__ __forceinline__ void encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
     // No difference at all: zero elimination leaves no byte, so RZE_1 emits
     // only its 2-byte trailer (the original chunk size).
     __syncthreads();
-    planes_read();
+    planes_read(2u);
     if (tid == 0) {
       lookback_publish(sy, sm.epoch, m.c, 2u);
-      pend = Pend{m.c, m.item, nw, 2, 0, 1};
-      *staged_byte(Y, 0, false) = (uint8_t)osize;
-      *staged_byte(Y, 1, false) = (uint8_t)(osize >> 8);
+      sm.pend = Pend{m.c, m.item, nw, 2, 0, 1, 1};
+      st_small[0] = (uint32_t)osize;
     }
-    return;
+    return false;
   }
 
   // Segment layout: thread t owns BIT-output words 32t..32t+31.
@@ -203,10 +204,10 @@ __device__ __forceinline__ void encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
   sm.l2[tid] = (uint16_t)K;
   uint32_t tot;
   const uint32_t ex = block_scan_excl(nz | (c1 << 16), sm.scan_a, tot);
-  planes_read();
   const uint32_t NZ = tot & 0xffffu, C1 = tot >> 16;
   const uint32_t zoff = ex & 0xffffu, c1off = ex >> 16;
-  // (barrier inside the scan: the planes have been read, Y may be overwritten)
+  planes_read(NZ + C1 + 288 + 6);
+  // (barrier inside the scan: the planes have been read)
 
   // Levels 2 and 3 and the top bitmap (d_REencode1wordperthread) from the
   // 256-byte level-2 bitmap: by warp 0, which publishes the size, and by every
@@ -214,7 +215,7 @@ __device__ __forceinline__ void encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
   bool raw = false;
   const bool close = NZ + C1 + 288 + 6 >= (unsigned)osize;
   const bool small = NZ + C1 + 288 + 6 <= SMALL;
-  uint32_t* st = small ? Y + CW : Y;
+  if (small) st = st_small;
   if (warp == 0 || close) {
     const uint2 b2 = reinterpret_cast<const uint2*>(sm.l2)[lane];
     const uint32_t pprev = __shfl_up_sync(0xffffffffu, b2.y >> 24, 1);
@@ -233,7 +234,7 @@ __device__ __forceinline__ void encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
     if (raw) csize = osize;
     if (tid == 0) {
       lookback_publish(sy, sm.epoch, m.c, csize);
-      pend = Pend{m.c, m.item, nw, (int)csize, raw ? -1 : (small ? CW : 0), 1};
+      sm.pend = Pend{m.c, m.item, nw, (int)csize, (int)raw, (int)small, 1};
     }
     if (warp == 0 && !raw) {
       if (NZ == 0) {
@@ -253,7 +254,7 @@ __device__ __forceinline__ void encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
       }
     }
   }
-  if (raw) return;
+  if (raw) return true;
   // Compaction of the zero-eliminated bytes and the kept level-1 bitmap bytes.
   if (small) {
     // few bytes, not padded: the non-zero words in order, read back from the
@@ -278,7 +279,7 @@ __device__ __forceinline__ void encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
       for (int j = 0; j < 16; j++)
         if ((K >> j) & 1) sb[p++] = (uint8_t)(M[j >> 2] >> (8 * (j & 3)));
     }
-    return;
+    return false;
   }
   if (__any_sync(0xffffffffu, nz != 0)) {
     pz = Packer(zoff);
@@ -290,23 +291,25 @@ __device__ __forceinline__ void encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
 #pragma unroll
     for (int j = 0; j < 4; j++) pk.put(st, M[j], pack_entry(K, j));
   }
+  return false;
 }
 
-// Writes out a pending chunk (p, output offset sm.payload_off, both visible
-// after a barrier) from its staging buffer -- or, for a raw chunk, from
+// Writes out the pending chunk (its output offset in sm.payload_off; both
+// visible after a barrier) from its staging buffer -- or, for a raw chunk, from
 // raw_word(w) -- and its size-table entry; the stream's last chunk also sets
 // the stream size.
 template <typename RawWord>
-__device__ __forceinline__ void flush_staged(const Ctl& sm, const Pend& p, const uint32_t* st, RawWord raw_word,
-                                             uint8_t* data_out, uint16_t* table_out, long long* out_size,
-                                             long long chunks) {
+__device__ __forceinline__ void flush_staged(const Ctl& sm, const uint32_t* st, const uint32_t* st_small,
+                                             RawWord raw_word, uint8_t* data_out, uint16_t* table_out,
+                                             long long* out_size, long long chunks) {
+  const Pend& p = sm.pend;
   const unsigned long long X = sm.payload_off;
-  const int nw = p.nw;
-  if (p.raw < 0) {
+  if (p.raw) {
+    const int nw = p.nw;
     store_payload(data_out + X, p.csize, [&](int w) -> uint32_t { return w < nw ? raw_word(w) : 0u; });
   } else {
-    st += p.raw;
-    const uint32_t pad = p.raw ? 31 : 5;
+    if (p.small) st = st_small;
+    const uint32_t pad = p.small ? 31 : 5;  // staged(), or no padding
     store_payload(data_out + X, p.csize, [&](int w) -> uint32_t { return st[(uint32_t)w + ((uint32_t)w >> pad)]; });
   }
   if (threadIdx.x == 0) {
@@ -317,18 +320,19 @@ __device__ __forceinline__ void flush_staged(const Ctl& sm, const Pend& p, const
 
 // The partial last chunk of a stream, out of line (it passes its words through
 // the calling thread's own row of Y, never through a pointer to the caller's
-// register array, which would put that array in local memory).  Ends with the
-// tails stored.
-__device__ __noinline__ void encode_partial(Ctl& sm, const Sync& sy, uint32_t prev0, uint32_t* Y, const StageMeta& m,
-                                            Pend& pend) {
+// register array, which would put that array in local memory).  The runs are
+// finished on return; returns whether the chunk is stored raw.
+__device__ __noinline__ bool encode_partial(Ctl& sm, const Sync& sy, uint32_t prev0, uint32_t* Y, uint32_t* st,
+                                            uint32_t* st_small, const StageMeta& m) {
   uint32_t w[32];
   row_load(Y, threadIdx.x, w);
   __syncthreads();  // Y becomes the plane buffer
   Packer pz(0), pk(0);
-  encode_chunk<false>(sm, sy, w, prev0, Y, m, pend, pz, pk, NoHook{}, NoHook{}, NoHook{});
+  const bool raw = encode_chunk<false>(sm, sy, w, prev0, Y, st, st_small, m, pz, pk, NoHook{}, NoHook{}, [](uint32_t) {});
   __syncthreads();
-  pz.finish(Y);
-  pk.finish(Y);
+  pz.finish(st);
+  pk.finish(st);
+  return raw;
 }
 
 }  // namespace cortado
