@@ -317,16 +317,15 @@ __device__ __forceinline__ void resolve_pending(Ctl& sm, const Src& src) {
 }
 // ... and writes it out from its staging buffer (every thread, after that
 // barrier).
-template <class Src, typename RawWord>
-__device__ __forceinline__ void write_pending(Ctl& sm, const Src& src, const uint32_t* st, const uint32_t* st_small,
-                                              RawWord raw_word) {
+// FLOATS: a raw chunk's payload is the input's floats, read again.
+template <bool FLOATS, class Src>
+__device__ __forceinline__ void write_pending(Ctl& sm, const Src& src, const uint32_t* st, const uint32_t* st_small) {
   const Pend& pd = sm.pend;
   if (!pd.valid) return;
   const OpArgs& Q = src.args(pd.item);
   const long long chunks = (Q.n + CS - 1) / CS;
-  const long long c = pd.c;
-  flush_staged(sm, st, st_small, [&](int w) -> uint32_t { return raw_word(Q, c, w); }, Q.out + HDR + 2 * chunks,
-               reinterpret_cast<uint16_t*>(Q.out + HDR), Q.out_size, chunks);
+  flush_staged(sm, st, st_small, FLOATS ? reinterpret_cast<const uint32_t*>(Q.in) + pd.c * (long long)CW : nullptr,
+               Q.out + HDR + 2 * chunks, reinterpret_cast<uint16_t*>(Q.out + HDR), Q.out_size, chunks);
 }
 
 // store (d_server_encode_kernel): floats -> SQ -> encode.  One buffer (A)
@@ -343,15 +342,11 @@ __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& 
   if (tid == 0) sm.pend.valid = 0;
   WalkState ws{-1};
   __syncthreads();
-  // a raw chunk stores the original floats, read again from global memory
-  auto raw_word = [](const OpArgs& Q, long long c, int w) -> uint32_t {
-    return reinterpret_cast<const uint32_t*>(Q.in)[c * (long long)CW + w];
-  };
   auto take = [&]() -> unsigned int { return (warp == LOADER && lane == 0) ? atomicAdd(&sy.counter[0], 1u) : 0u; };
   auto load = [&](int t, unsigned int g) {
     if (warp == LOADER) prefetch_floats(sm, t, __shfl_sync(0xffffffffu, g, 0), src, ws);
   };
-  auto flush = [&](int t) { write_pending(sm, src, stage_buf(sm, t), stage_buf(sm, t) + CW, raw_word); };
+  auto flush = [&](int t) { write_pending<true>(sm, src, stage_buf(sm, t), stage_buf(sm, t) + CW); };
   load(0, take());
   int s = 0;  // this chunk's buffer and slots; also the barrier's phase
   for (;; s ^= 1) {
@@ -392,7 +387,7 @@ __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& 
     if (full) {
       unsigned int g = 0;
       Packer pz(0), pk(0);
-      encode_chunk<true>(
+      encode_chunk<true, true>(
           sm, A_.sy, v, prev0, A, A, A + CW, m, pz, pk, [&]() { resolve_pending(sm, src); },
           [&]() {
             g = take();
@@ -656,23 +651,24 @@ __device__ __forceinline__ void client_apply(const OpArgs& A, long long c, int n
 }
 
 // init_send with apply, for a chunk stored uncompressed: its bins (rebuilt
-// into row tid of Yw by raw_rebuild) replace the dequantized words this
+// into words 32 tid .. of Yw by raw_rebuild) replace the dequantized words this
 // thread wrote, as init_recv emits a raw chunk's bins unchanged.
 __device__ __noinline__ void client_raw_bins(const OpArgs& A, long long c, int nw, const uint32_t* Yw) {
   const int tid = threadIdx.x;
   uint32_t* row = reinterpret_cast<uint32_t*>(A.client) + c * (long long)CW + 32 * tid;
   for (int k = 0; k < 32; k++)
-    if (32 * tid + k < nw) row[k] = Yw[swz(32 * tid + k)];
+    if (32 * tid + k < nw) row[k] = Yw[32 * tid + k];
 }
 
 // Rebuilds a raw chunk's requantized words from the plane buffer into the
-// staging buffer (out of line: only chunks that do not compress take it, and
-// the re-encoders' loop is large enough to stall on instruction fetch).
+// staging buffer, in order (out of line: only chunks that do not compress take
+// it, and the re-encoders' loop is large enough to stall on instruction fetch).
 __device__ __noinline__ void raw_rebuild(Ctl& sm, const uint32_t* X, int nw, uint32_t* Yw) {
   uint32_t w[32], before;
-  if (nw == CW) planes_to_words<true>(sm, X, nw, w, before);
-  else planes_to_words<false>(sm, X, nw, w, before);
-  row_store(Yw, threadIdx.x, w);
+  if (nw == CW) planes_to_words<true, true>(sm, X, nw, w, before);
+  else planes_to_words<false, true>(sm, X, nw, w, before);
+#pragma unroll
+  for (int k = 0; k < 32; k++) Yw[32 * threadIdx.x + k] = w[k];
 }
 
 // Blocking flush of the re-encoders' pending chunk, outside the hot path: when
@@ -683,7 +679,7 @@ __device__ __noinline__ void flush_now(Ctl& sm, const Src src, uint32_t* R) {
   __syncthreads();
   resolve_pending(sm, src);
   __syncthreads();
-  write_pending(sm, src, R, R, [R](const OpArgs&, long long, int w) -> uint32_t { return R[swz(w)]; });
+  write_pending<false>(sm, src, R, R);
   __syncthreads();
   if (threadIdx.x == 0) sm.pend.valid = 0;
 }
@@ -701,8 +697,10 @@ __device__ __noinline__ void flush_now(Ctl& sm, const Src src, uint32_t* R) {
 // (Decoding in place in one buffer and staging in the other took 11 barriers a
 // chunk; this takes 7.  256 MiB: init_send 462 -> 320 us and resi_send 468 ->
 // 340 us on sinusoids with noise, 552 -> 414 and 516 -> 387 us on dense data,
-// 269 -> 256 and 282 -> 277 us on nearly all zero bins.  Instruction fetch is
-// now the largest stall.)
+// 269 -> 256 and 282 -> 277 us on nearly all zero bins.  Instruction fetch was
+// then the largest stall; the loops of planes_to_words, rze_decode and
+// encode_chunk that are not unrolled brought init_send to 294, 373 and 245 us,
+// resi_send to 320, 370 and 266 us.)
 // APPLY: the fused send-and-apply forms (items with a client's floats); the
 // plain forms are compiled without that code.
 constexpr int ROOM = (2 * BUF_WORDS - CW) * 4;  // bytes of R
@@ -759,7 +757,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
 #pragma unroll
       for (int k = 0; k < 32; k++) v[k] = 0;
     } else if (full && kind == CHUNK_PLANES) {
-      planes_to_words<true>(sm, Y, CW, v, before);
+      planes_to_words<true, true>(sm, Y, CW, v, before);
     } else {
       row_load(Y, tid, v);
       if (!full && 32 * tid + 32 > m.nw) {
@@ -822,15 +820,13 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
     if (full) {
       __syncthreads();  // the rows of Y are free
       Packer pz(0), pk(0);
-      raw_out = encode_chunk<true>(
+      raw_out = encode_chunk<true, false>(
           sm, A.sy, v, before, Y, R, R, m, pz, pk,
           [&]() {
             resolve_pending(sm, src);
             park(s ^ 1);
           },
-          [&]() {
-            write_pending(sm, src, R, R, [R](const OpArgs&, long long, int w) -> uint32_t { return R[swz(w)]; });
-          },
+          [&]() { write_pending<false>(sm, src, R, R); },
           [&](uint32_t bytes) {
             if (feeder) {
               const int cs = min(sm.st[s ^ 1].csize, CS);
@@ -935,7 +931,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
       for (int k = 0; k < 32; k++) v[k] = 0;
     } else if (full && kind == CHUNK_PLANES) {
       uint32_t before;
-      planes_to_words<true>(sm, Q, CW, v, before);
+      planes_to_words<true, false>(sm, Q, CW, v, before);
     } else {
       row_load(Q, tid, v);
     }

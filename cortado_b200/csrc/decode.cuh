@@ -204,25 +204,36 @@ __device__ __forceinline__ ChunkKind rze_decode(Ctl& sm, const Sync& sy, const S
     // Every word, two at a time, each lane starting at another pair (lane / 2):
     // lanes' bytes are up to 128 bytes apart, and in the same order their
     // reads would fall into the same banks.  R: the mask rotated to that start.
+    // (A loop over four words of the mask: unrolled whole, it made every kernel
+    // slower on dense data, init_recv of 256 MiB at 25% 157 -> 164 us, and the
+    // re-encoders stall on instruction fetch.)
     const uint32_t rot = ((uint32_t)lane >> 1) * 2;
     uint32_t R[4];
     rot_nibbles(M, rot, R);
-    p += nibble_prefix(M, rot);
+    p += rot ? nibble_prefix(M, rot) : nz;
+    uint32_t k = rot;
+#pragma unroll 1
+    for (int i = 0; i < 4; i++) {
+      const uint32_t r = R[0];
+      R[0] = R[1];
+      R[1] = R[2];
+      R[2] = R[3];
 #pragma unroll
-    for (int j = 0; j < 32; j += 2) {
-      const uint32_t k = (rot + j) & 30u;
-      if (j && k == 0) p -= nz;
-      const uint32_t mk = prmt(R[j >> 3], 0u, 0x4440u | ((j >> 1) & 3));
-      uint32_t s0, s1;
-      spread_sel2(mk, s0, s1);
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(st + (p & ~3u));
-      uint2 q;
-      q.x = prmt(__funnelshift_r(w[0], w[1], 8 * p), 0u, s0);
-      p += __popc(mk & 15u);
-      w = reinterpret_cast<const uint32_t*>(st + (p & ~3u));
-      q.y = prmt(__funnelshift_r(w[0], w[1], 8 * p), 0u, s1);
-      p += __popc(mk >> 4);
-      *reinterpret_cast<uint2*>(row + (k ^ (xr << 2))) = q;
+      for (int j = 0; j < 4; j++) {
+        if (k == 0) p -= nz;  // back to the first word's bytes
+        const uint32_t mk = prmt(r, 0u, 0x4440u | j);
+        uint32_t s0, s1;
+        spread_sel2(mk, s0, s1);
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(st + (p & ~3u));
+        uint2 q;
+        q.x = prmt(__funnelshift_r(w[0], w[1], 8 * p), 0u, s0);
+        p += __popc(mk & 15u);
+        w = reinterpret_cast<const uint32_t*>(st + (p & ~3u));
+        q.y = prmt(__funnelshift_r(w[0], w[1], 8 * p), 0u, s1);
+        p += __popc(mk >> 4);
+        *reinterpret_cast<uint2*>(row + (k ^ (xr << 2))) = q;
+        k = (k + 2) & 30u;
+      }
     }
   }
   __syncthreads();
@@ -241,7 +252,7 @@ __device__ __noinline__ ChunkKind decode_partial(Ctl& sm, const Sync& sy, const 
   if (kind != CHUNK_PLANES) return kind;
   uint32_t w[32];
   uint32_t before;
-  planes_to_words<false>(sm, Q, m.nw, w, before);
+  planes_to_words<false, true>(sm, Q, m.nw, w, before);
   row_store(Q, threadIdx.x, w);
   return kind;
 }

@@ -306,22 +306,11 @@ __device__ __forceinline__ void transpose32(uint32_t (&a)[32]) {
   }
   transpose_blocks(a);
 }
-// The same for 32 words below 2^16 (planes 0..15 are zero): words k and k + 16
-// share a register, so the stages run on 16 registers, which end up as planes
-// 16..31; and back.  128 and 112 instructions fewer than transpose32.
-__device__ __forceinline__ void narrow_to_planes(const uint32_t (&a)[32], uint32_t (&p)[16]) {
-#pragma unroll
-  for (int k = 0; k < 16; k++) p[k] = __byte_perm(a[k], a[k + 16], 0x1054);
-  transpose_blocks(p);
-}
-__device__ __forceinline__ void planes_to_narrow(uint32_t (&p)[16], uint32_t (&a)[32]) {
-  transpose_blocks(p);
-#pragma unroll
-  for (int k = 0; k < 16; k++) {
-    a[k] = p[k] >> 16;
-    a[k + 16] = p[k] & 0xffffu;
-  }
-}
+// Full groups are transposed one half of the planes at a time: words k and
+// k + 16 share a register (their high halves for planes 0..15, their low halves
+// for planes 16..31), and the stages run on 16 registers.  The pass for planes
+// that are zero in the whole warp is left out, and both passes are the same
+// code, half as long as transpose32.
 
 // ---------------------------------------------------------------- byte masks
 // 4-bit mask of the non-zero bytes of x (bit b <-> byte b).

@@ -99,7 +99,10 @@ struct Packer {
 // which the planes are read, planes_ready() after it, and planes_read(n) after
 // the next one, with a bound n of the payload's bytes.
 // FULL: a whole 16 KiB chunk (nw == 4096), with compile-time addressing.
-template <bool FULL, typename Written, typename Ready, typename Read>
+// KEEP: the plane words stay in registers (st is Y, or a partial chunk); else
+// they are read again for the packing, eight at a time in a loop, which keeps
+// the re-encoders' code short.
+template <bool FULL, bool KEEP, typename Written, typename Ready, typename Read>
 __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (&v)[32], uint32_t prev0, uint32_t* Y,
                                              uint32_t* st, uint32_t* st_small, const StageMeta& m, Packer& pz, Packer& pk,
                                              Written planes_written, Ready planes_ready, Read planes_read) {
@@ -128,18 +131,21 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
     const uint32_t bits = __reduce_or_sync(0xffffffffu, any);
     uint32_t pe, po;
     plane_offsets(tid, pe, po);
-    if (bits >= 0x10000u) {
-      transpose32(v);
-#pragma unroll
-      for (int s = 0; s < 32; s++) Y[128 * s + ((s & 1) ? po : pe)] = v[s];
-    } else {  // planes 0..15 are zero (and the others too when no word differs)
+    int half = 0;
+    if (bits < 0x10000u) {  // planes 0..15 are zero: lanes 2s and 2s + 1 clear row s
+      half = 1;
       uint4* r = reinterpret_cast<uint4*>(Y + 32 * (4 * (lane >> 1) + warp));
 #pragma unroll
       for (int u = 0; u < 4; u++) r[((lane & 1) << 2 | u) ^ ((lane >> 1) & 7)] = make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll 1
+    for (; half < 2; half++) {
       uint32_t p[16];
-      narrow_to_planes(v, p);
 #pragma unroll
-      for (int s = 0; s < 16; s++) Y[128 * (16 + s) + ((s & 1) ? po : pe)] = p[s];
+      for (int k = 0; k < 16; k++) p[k] = prmt(v[k], v[k + 16], half ? 0x1054u : 0x3276u);
+      if (bits) transpose_blocks(p);
+#pragma unroll
+      for (int s = 0; s < 16; s++) Y[2048 * half + 128 * s + ((s & 1) ? po : pe)] = p[s];
     }
   } else if (tid < G) {
     transpose32(v);
@@ -167,21 +173,38 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
   }
 
   // Segment layout: thread t owns BIT-output words 32t..32t+31.
-  uint32_t q[32];
-  row_load(Y, tid, q);
-  if (!FULL && 32 * tid + 32 > nw) {
-#pragma unroll
-    for (int k = 0; k < 32; k++)
-      if (32 * tid + k >= nw) q[k] = 0;
-  }
   // Zero-elimination bitmap (d_ZEencodebyteshort): bit i <-> byte i != 0.
-  uint32_t M[4] = {0, 0, 0, 0};
-  uint32_t qany = 0;
+  uint32_t q[32], M[4] = {0, 0, 0, 0};
+  auto load8 = [&](int j, uint32_t* x) {
+    const uint4* r = reinterpret_cast<const uint4*>(Y + 32 * tid);
+    const uint4 a = r[(2 * j) ^ (tid & 7)], b = r[(2 * j + 1) ^ (tid & 7)];
+    x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+  };
+  if (KEEP) {
+    row_load(Y, tid, q);
+    if (!FULL && 32 * tid + 32 > nw) {
 #pragma unroll
-  for (int k = 0; k < 32; k++) qany |= q[k];
-  if (qany) {
+      for (int k = 0; k < 32; k++)
+        if (32 * tid + k >= nw) q[k] = 0;
+    }
+    uint32_t qany = 0;
 #pragma unroll
-    for (int j = 0; j < 4; j++) M[j] = nz_bytes8(q + 8 * j);
+    for (int k = 0; k < 32; k++) qany |= q[k];
+    if (qany) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) M[j] = nz_bytes8(q + 8 * j);
+    }
+  } else {
+#pragma unroll 1
+    for (int j = 0; j < 4; j++) {
+      uint32_t x[8];
+      load8(j, x);
+      M[0] = M[1];
+      M[1] = M[2];
+      M[2] = M[3];
+      M[3] = 0;
+      if (x[0] | x[1] | x[2] | x[3] | x[4] | x[5] | x[6] | x[7]) M[3] = nz_bytes8(x);
+    }
   }
   const uint32_t nz = __popc(M[0]) + __popc(M[1]) + __popc(M[2]) + __popc(M[3]);
   // Last bitmap byte of the previous segment (RE's predecessor of byte 0).
@@ -281,35 +304,52 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
     }
     return false;
   }
-  if (__any_sync(0xffffffffu, nz != 0)) {
+  if (__any_sync(0xffffffffu, (nz | K) != 0)) {
     pz = Packer(zoff);
-#pragma unroll
-    for (int k = 0; k < 32; k++) pz.put(st, q[k], pack_entry(M[k >> 3], k & 7));
-  }
-  if (__any_sync(0xffffffffu, K != 0)) {
     pk = Packer(NZ + c1off);
+    if (KEEP) {
 #pragma unroll
-    for (int j = 0; j < 4; j++) pk.put(st, M[j], pack_entry(K, j));
+      for (int k = 0; k < 32; k++) pz.put(st, q[k], pack_entry(M[k >> 3], k & 7));
+#pragma unroll
+      for (int j = 0; j < 4; j++) pk.put(st, M[j], pack_entry(K, j));
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < 4; j++) {
+        uint32_t x[8];
+        load8(j, x);
+        const uint32_t m4 = M[0];
+        M[0] = M[1];
+        M[1] = M[2];
+        M[2] = M[3];
+#pragma unroll
+        for (int k = 0; k < 8; k++) pz.put(st, x[k], pack_entry(m4, k));
+        pk.put(st, m4, pack_entry(K, 0));
+        K >>= 4;
+      }
+    }
   }
   return false;
 }
 
+// A raw chunk's payload from words in global memory (out of line: rare).
+__device__ __noinline__ void flush_words(uint8_t* dst, const uint32_t* words, int nw) {
+  store_payload(dst, 4 * nw, [=](int w) -> uint32_t { return w < nw ? words[w] : 0u; });
+}
+
 // Writes out the pending chunk (its output offset in sm.payload_off; both
 // visible after a barrier) from its staging buffer -- or, for a raw chunk, from
-// raw_word(w) -- and its size-table entry; the stream's last chunk also sets
-// the stream size.
-template <typename RawWord>
+// raw_words, when not null (else its words are staged too, not padded) -- and
+// its size-table entry; the stream's last chunk also sets the stream size.
 __device__ __forceinline__ void flush_staged(const Ctl& sm, const uint32_t* st, const uint32_t* st_small,
-                                             RawWord raw_word, uint8_t* data_out, uint16_t* table_out,
+                                             const uint32_t* raw_words, uint8_t* data_out, uint16_t* table_out,
                                              long long* out_size, long long chunks) {
   const Pend& p = sm.pend;
   const unsigned long long X = sm.payload_off;
-  if (p.raw) {
-    const int nw = p.nw;
-    store_payload(data_out + X, p.csize, [&](int w) -> uint32_t { return w < nw ? raw_word(w) : 0u; });
+  if (p.raw && raw_words) {
+    flush_words(data_out + X, raw_words, p.nw);
   } else {
     if (p.small) st = st_small;
-    const uint32_t pad = p.small ? 31 : 5;  // staged(), or no padding
+    const uint32_t pad = (p.small | p.raw) ? 31 : 5;  // no padding, or staged()
     store_payload(data_out + X, p.csize, [&](int w) -> uint32_t { return st[(uint32_t)w + ((uint32_t)w >> pad)]; });
   }
   if (threadIdx.x == 0) {
@@ -328,7 +368,7 @@ __device__ __noinline__ bool encode_partial(Ctl& sm, const Sync& sy, uint32_t pr
   row_load(Y, threadIdx.x, w);
   __syncthreads();  // Y becomes the plane buffer
   Packer pz(0), pk(0);
-  const bool raw = encode_chunk<false>(sm, sy, w, prev0, Y, st, st_small, m, pz, pk, NoHook{}, NoHook{}, [](uint32_t) {});
+  const bool raw = encode_chunk<false, true>(sm, sy, w, prev0, Y, st, st_small, m, pz, pk, NoHook{}, NoHook{}, [](uint32_t) {});
   __syncthreads();
   pz.finish(st);
   pk.finish(st);

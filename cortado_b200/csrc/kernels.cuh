@@ -218,8 +218,9 @@ __device__ __forceinline__ void rot_nibbles(const uint32_t (&M)[4], int r, uint3
 // prefix sum plus a block scan of the group totals), and returns the group's
 // words in v[32] (words at or beyond nw are 0) and the word before them in
 // `before` (0 for the first group).  Ends with a barrier (the scan's), after
-// which the plane buffer may be reused.
-template <bool FULL>
+// which the plane buffer may be reused.  SHORT: loops are not unrolled (the
+// re-encoders, whose code is long).
+template <bool FULL, bool SHORT>
 __device__ __forceinline__ void planes_to_words(Ctl& sm, const uint32_t* plane, int nw_in, uint32_t (&v)[32],
                                                 uint32_t& before) {
   const int tid = threadIdx.x;
@@ -230,27 +231,28 @@ __device__ __forceinline__ void planes_to_words(Ctl& sm, const uint32_t* plane, 
   if (FULL) {
     uint32_t pe, po;
     plane_offsets(tid, pe, po);
-    uint32_t p[16], high = 0, any = 0;
+    uint32_t h[16], p[16];  // planes 0..15 and 16..31, transposed
 #pragma unroll
-    for (int s = 0; s < 16; s++) {
-      v[s] = plane[128 * s + ((s & 1) ? po : pe)];
-      high |= v[s];
+    for (int s = 0; s < 16; s++) p[s] = 0;
+    live = false;
+#pragma unroll(SHORT ? 1 : 2)
+    for (int half = 0; half < 2; half++) {
+      uint32_t any = 0;
+#pragma unroll
+      for (int s = 0; s < 16; s++) {
+        h[s] = p[s];
+        p[s] = plane[2048 * half + 128 * s + ((s & 1) ? po : pe)];
+        any |= p[s];
+      }
+      if (__any_sync(0xffffffffu, any != 0)) {
+        transpose_blocks(p);
+        live = true;
+      }
     }
 #pragma unroll
-    for (int s = 0; s < 16; s++) {
-      p[s] = plane[128 * (16 + s) + ((s & 1) ? po : pe)];
-      any |= p[s];
-    }
-    if (__any_sync(0xffffffffu, high != 0)) {
-#pragma unroll
-      for (int s = 0; s < 16; s++) v[16 + s] = p[s];
-      transpose32(v);
-    } else {
-      live = __any_sync(0xffffffffu, any != 0);  // zero planes transpose to zero words
-      if (live) planes_to_narrow(p, v);
-      else
-#pragma unroll
-        for (int s = 0; s < 16; s++) v[16 + s] = 0;
+    for (int k = 0; k < 16; k++) {
+      v[k] = __byte_perm(p[k], h[k], 0x7632);
+      v[k + 16] = __byte_perm(p[k], h[k], 0x5410);
     }
   } else if (tid < G) {
 #pragma unroll
