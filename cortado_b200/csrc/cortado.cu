@@ -355,7 +355,6 @@ __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& 
     if (m.g >= src.total) break;
     uint32_t* A = stage_buf(sm, s);
     const OpArgs& A_ = src.args(m.item);
-    const bool full = m.nw == CW;
     if (!m.tma) {
       load_plain_rows(A, A_.in, m.c, m.nw);
       __syncthreads();
@@ -384,28 +383,18 @@ __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& 
       }
     }
     __syncthreads();  // A has been read; the pending payload is complete
-    if (full) {
-      unsigned int g = 0;
-      Packer pz(0), pk(0);
-      encode_chunk<true, true>(
-          sm, A_.sy, v, prev0, A, A, A + CW, m, pz, pk, [&]() { resolve_pending(sm, src); },
-          [&]() {
-            g = take();
-            flush(s ^ 1);
-          },
-          [&](uint32_t) { load(s ^ 1, g); });
-      __syncthreads();  // the payload's full words are in place
-      pz.finish(A);
-      pk.finish(A);
-    } else {
-      row_store(A, tid, v);
-      resolve_pending(sm, src);
-      __syncthreads();
-      flush(s ^ 1);
-      __syncthreads();
-      encode_partial(sm, A_.sy, prev0, A, A, A + CW, m);
-      load(s ^ 1, take());
-    }
+    unsigned int g = 0;
+    Packer pz(0), pk(0);
+    encode_chunk<true>(
+        sm, A_.sy, v, prev0, A, A, A + CW, m, pz, pk, [&]() { resolve_pending(sm, src); },
+        [&]() {
+          g = take();
+          flush(s ^ 1);
+        },
+        [&](uint32_t) { load(s ^ 1, g); });
+    __syncthreads();  // the payload's full words are in place
+    pz.finish(A);
+    pk.finish(A);
   }
   resolve_pending(sm, src);
   __syncthreads();
@@ -568,6 +557,14 @@ __device__ __forceinline__ void issue_stream(Ctl& sm, int t, const Src& src, uin
 // client word, no lossless bin), else the per-word forms, as in the decoders.
 // A partial chunk works word by word on the client's floats directly.
 template <int OP>
+__device__ __noinline__ void client_apply_partial(uint32_t* client, int nw, Quant q, const uint32_t* X) {
+  const FastQ fq = make_fastq(q.eb_e);
+  for (int w = 32 * threadIdx.x; w < min(32 * (int)threadIdx.x + 32, nw); w++) {
+    const uint32_t b = X[swz(w)];
+    client[w] = (OP == OP_S2C) ? iq_mixed(b, fq, q) : iq_mixed(cq_mixed(client[w], fq, q) + b, fq, q);
+  }
+}
+template <int OP>
 __device__ __forceinline__ void client_apply(const OpArgs& A, long long c, int nw, const uint32_t (&v)[32], Quant q,
                                              uint32_t* X) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -640,13 +637,8 @@ __device__ __forceinline__ void client_apply(const OpArgs& A, long long c, int n
     }
     __syncwarp();  // the rows are read before the encoder reuses the buffer
   } else {
-    uint32_t* row = reinterpret_cast<uint32_t*>(A.client) + c * (long long)CW + 32 * tid;
-#pragma unroll
-    for (int k = 0; k < 32; k++) {
-      if (32 * tid + k < nw) {
-        row[k] = (OP == OP_S2C) ? iq_mixed(v[k], fq, q) : iq_mixed(cq_mixed(row[k], fq, q) + v[k], fq, q);
-      }
-    }
+    row_store(X, tid, v);
+    client_apply_partial<OP>(reinterpret_cast<uint32_t*>(A.client) + c * (long long)CW, nw, q, X);
   }
 }
 
@@ -663,17 +655,16 @@ __device__ __noinline__ void client_raw_bins(const OpArgs& A, long long c, int n
 // Rebuilds a raw chunk's requantized words from the plane buffer into the
 // staging buffer, in order (out of line: only chunks that do not compress take
 // it, and the re-encoders' loop is large enough to stall on instruction fetch).
-__device__ __noinline__ void raw_rebuild(Ctl& sm, const uint32_t* X, int nw, uint32_t* Yw) {
+__device__ __noinline__ void raw_rebuild(Ctl& sm, uint32_t* X, int nw, uint32_t* Yw) {
   uint32_t w[32], before;
-  if (nw == CW) planes_to_words<true, true>(sm, X, nw, w, before);
-  else planes_to_words<false, true>(sm, X, nw, w, before);
+  if (nw != CW) widen_planes(X, nw);
+  planes_to_words<true>(sm, X, w, before);
 #pragma unroll
   for (int k = 0; k < 32; k++) Yw[32 * threadIdx.x + k] = w[k];
 }
 
 // Blocking flush of the re-encoders' pending chunk, outside the hot path: when
-// the next payload does not fit beside it, around partial chunks and at the end
-// of the loop.  Every earlier write to R may precede it without a barrier.
+// the next payload does not fit beside it and at the end of the loop.  Every earlier write to R may precede it without a barrier.
 template <class Src>
 __device__ __noinline__ void flush_now(Ctl& sm, const Src src, uint32_t* R) {
   __syncthreads();
@@ -741,9 +732,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
     const StageMeta& m = sm.st[s];
     if (m.g >= src.total) break;
     const OpArgs& A = src.args(m.item);
-    const bool full = m.nw == CW;
-    const ChunkKind kind =
-        full ? rze_decode<true>(sm, A.sy, m, R, Y, NoHook{}) : decode_partial(sm, A.sy, m, R, Y, NoHook{});
+    const ChunkKind kind = rze_decode(sm, A.sy, m, R, Y, NoHook{});
     const unsigned int g = take();
     if (m.bad >= 2) {  // unusable stream header (batched): nothing to write
       resolve(s ^ 1, g);
@@ -756,16 +745,11 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
     if (kind == CHUNK_ZERO) {
 #pragma unroll
       for (int k = 0; k < 32; k++) v[k] = 0;
-    } else if (full && kind == CHUNK_PLANES) {
-      planes_to_words<true, true>(sm, Y, CW, v, before);
+    } else if (kind == CHUNK_PLANES) {
+      planes_to_words<true>(sm, Y, v, before);
     } else {
       row_load(Y, tid, v);
-      if (!full && 32 * tid + 32 > m.nw) {
-#pragma unroll
-        for (int k = 0; k < 32; k++)
-          if (32 * tid + k >= m.nw) v[k] = 0;
-      }
-      before = (tid && 32 * tid - 1 < m.nw) ? Y[swz(32 * tid - 1)] : 0u;
+      before = tid ? Y[swz(32 * tid - 1)] : 0u;
       __syncthreads();  // rows are scratch from here on
     }
     {
@@ -816,40 +800,31 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
       resolve(s ^ 1, g);
       if (APPLY && A.client) client_apply<OP>(A, m.c, m.nw, v, OP == OP_S2C ? q1 : q2, Y);
     }
-    bool raw_out, held;
-    if (full) {
-      __syncthreads();  // the rows of Y are free
-      Packer pz(0), pk(0);
-      raw_out = encode_chunk<true, false>(
-          sm, A.sy, v, before, Y, R, R, m, pz, pk,
-          [&]() {
-            resolve_pending(sm, src);
-            park(s ^ 1);
-          },
-          [&]() { write_pending<false>(sm, src, R, R); },
-          [&](uint32_t bytes) {
-            if (feeder) {
-              const int cs = min(sm.st[s ^ 1].csize, CS);
-              const bool fits = room_out(min((int)bytes, CS)) + room_in(cs) <= ROOM;
-              if (lane == 0) sm.held = !fits;
-              if (fits) issue(s ^ 1);
-            }
-          });
-      if (raw_out) raw_rebuild(sm, Y, CW, R);
-      __syncthreads();  // the payload's full words are in place
-      pz.finish(R);
-      pk.finish(R);
-      held = sm.held;
-    } else {
-      park(s ^ 1);
-      flush_now(sm, src, R);
-      row_store(Y, tid, v);
-      raw_out = encode_partial(sm, A.sy, before, Y, R, R, m);
-      if (raw_out) raw_rebuild(sm, Y, m.nw, R);
-      held = true;
+    __syncthreads();  // the rows of Y are free
+    Packer pz(0), pk(0);
+    const bool raw_out = encode_chunk<false>(
+        sm, A.sy, v, before, Y, R, R, m, pz, pk,
+        [&]() {
+          resolve_pending(sm, src);
+          park(s ^ 1);
+        },
+        [&]() { write_pending<false>(sm, src, R, R); },
+        [&](uint32_t bytes) {
+          if (feeder) {
+            const int cs = min(sm.st[s ^ 1].csize, CS);
+            const bool fits = room_out(min((int)bytes, CS)) + room_in(cs) <= ROOM;
+            if (lane == 0) sm.held = !fits;
+            if (fits) issue(s ^ 1);
+          }
+        });
+    if (raw_out) {
+      raw_rebuild(sm, Y, m.nw, R);
+      if (OP == OP_S2C && APPLY && A.client) client_raw_bins(A, m.c, m.nw, R);
     }
-    if (raw_out && OP == OP_S2C && APPLY && A.client) client_raw_bins(A, m.c, m.nw, R);
-    if (held) {
+    __syncthreads();  // the payload's full words are in place
+    pz.finish(R);
+    pk.finish(R);
+    if (sm.held) {
       flush_now(sm, src, R);
       if (feeder) issue(s ^ 1);
     }
@@ -907,7 +882,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     auto q_free = [&]() {
       if (tid == TMA_TID) bulk_wait_read();  // the previous chunk's TMA store has read Q
     };
-    const ChunkKind kind = full ? rze_decode<true>(sm, A.sy, m, P, Q, q_free) : decode_partial(sm, A.sy, m, P, Q, q_free);
+    const ChunkKind kind = rze_decode(sm, A.sy, m, P, Q, q_free);
     if (feeder) {
       park_stream(sm, s ^ 1, src, ah);
       issue_stream(sm, s ^ 1, src, reinterpret_cast<uint8_t*>(P), 0);
@@ -929,9 +904,9 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     if (kind == CHUNK_ZERO) {
 #pragma unroll
       for (int k = 0; k < 32; k++) v[k] = 0;
-    } else if (full && kind == CHUNK_PLANES) {
+    } else if (kind == CHUNK_PLANES) {
       uint32_t before;
-      planes_to_words<true, false>(sm, Q, CW, v, before);
+      planes_to_words<false>(sm, Q, v, before);
     } else {
       row_load(Q, tid, v);
     }
@@ -940,7 +915,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     if (OP == OP_RAPPLY) {
       // d_iRESI_4 (d_RESI_4.h:79-94): requantize the client's floats to the
       // destination bound, add the residual, dequantize.
-      if (!full || kind != CHUNK_PLANES) __syncthreads();  // sm.src_side; Q has been read
+      if (kind != CHUNK_PLANES) __syncthreads();  // sm.src_side; Q has been read
       const uint32_t* S = Q;  // where the client's chunk is
       if (full && A.has_map_in) {
         if (sm.src_side) {
@@ -1375,8 +1350,11 @@ Sync next_sync(cortado_ctx* ctx, cudaStream_t, int op = 0) {
   return s;
 }
 
+// A CTA per chunk, and one more for the helper (a one-chunk launch has none), up
+// to the persistent grid.  (Without the helper's own CTA, one CTA of a small
+// launch worked on two chunks, one after the other.)
 int grid_for(int per_sm_grid, int64_t chunks) {
-  long long g = chunks < 1 ? 1 : chunks;
+  const long long g = chunks < 2 ? 1 : chunks + 1;
   return (int)(g < per_sm_grid ? g : per_sm_grid);
 }
 

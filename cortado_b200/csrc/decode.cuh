@@ -76,7 +76,8 @@ enum ChunkKind : int { CHUNK_ZERO = 0, CHUNK_PLANES = 1, CHUNK_RAW = 2 };
 
 // Undoes RZE_1 (d_iRZE, d_RZE.h:127-206) for the chunk whose payload the
 // stage's loads brought into P (at byte offset m.d, m.csize bytes): the BIT_4
-// output goes to the swizzled plane buffer Q.  Returns CHUNK_PLANES,
+// output goes to the swizzled plane buffer Q (a partial chunk's in the full
+// chunks' places).  Returns CHUNK_PLANES,
 // CHUNK_ZERO (all words are zero, also for a chunk that cannot be decoded;
 // Q is not written) or CHUNK_RAW (Q holds the words as stored, in the float
 // tiles' swizzle).  q_free() runs on every thread before the barrier after
@@ -86,11 +87,11 @@ enum ChunkKind : int { CHUNK_ZERO = 0, CHUNK_PLANES = 1, CHUNK_RAW = 2 };
 // 90 instructions), so no warp waits for another before the level-1 bitmap
 // (warp 0 decoding them for the others took a barrier and left three warps
 // idle meanwhile).
-template <bool FULL, typename Free>
+template <typename Free>
 __device__ __forceinline__ ChunkKind rze_decode(Ctl& sm, const Sync& sy, const StageMeta& m, const uint32_t* P,
                                                 uint32_t* Q, Free q_free) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nw = FULL ? CW : m.nw;
+  const int nw = m.nw;
   const int osize = nw * 4;
   const uint8_t* st = reinterpret_cast<const uint8_t*>(P);
   const int csize = m.csize, d = m.d;
@@ -107,7 +108,7 @@ __device__ __forceinline__ ChunkKind rze_decode(Ctl& sm, const Sync& sy, const S
     for (int j = 0; j < 32; j++) {
       const int w = tid + NT * j;
       const int o = d + 4 * w;
-      if (FULL || w < nw) Q[swz(w)] = __funnelshift_r(P[o >> 2], P[(o >> 2) + 1], 8 * (o & 3));
+      if (w < nw) Q[swz(w)] = __funnelshift_r(P[o >> 2], P[(o >> 2) + 1], 8 * (o & 3));
     }
     __syncthreads();
     return CHUNK_RAW;
@@ -158,15 +159,14 @@ __device__ __forceinline__ ChunkKind rze_decode(Ctl& sm, const Sync& sy, const S
     }
   }
   ok = ok && wok;
-  // bitmap bits beyond the chunk must be clear
-  if (!FULL && 32 * tid + 32 > nw) {
+  if (32 * tid + 32 > nw) {  // bitmap bits beyond the chunk must be clear
 #pragma unroll
-    for (int k = 0; k < 32; k++)
-      if (32 * tid + k >= nw) {
-        const uint32_t bm = 15u << (4 * (k & 7));
-        if (M[k >> 3] & bm) ok = false;
-        M[k >> 3] &= ~bm;
-      }
+    for (int j = 0; j < 4; j++) {
+      const int keep = 4 * (nw - 32 * tid) - 32 * j;
+      const uint32_t k = keep >= 32 ? 0xffffffffu : keep <= 0 ? 0u : (1u << keep) - 1u;
+      if (M[j] & ~k) ok = false;
+      M[j] &= k;
+    }
   }
   q_free();
   const uint32_t nz = __popc(M[0]) + __popc(M[1]) + __popc(M[2]) + __popc(M[3]);
@@ -237,24 +237,8 @@ __device__ __forceinline__ ChunkKind rze_decode(Ctl& sm, const Sync& sy, const S
     }
   }
   __syncthreads();
+  if (nw != CW) widen_planes(Q, nw);
   return CHUNK_PLANES;
-}
-
-// The partial last chunk of a stream runs out of line, so the full chunks'
-// loop stays small for the instruction caches; its words pass through the
-// calling thread's own row of Q (taking the address of the caller's register
-// array would put it in local memory).  Returns the chunk's kind; the words
-// are in Q unless it is CHUNK_ZERO.
-template <typename Free>
-__device__ __noinline__ ChunkKind decode_partial(Ctl& sm, const Sync& sy, const StageMeta& m, const uint32_t* P,
-                                                 uint32_t* Q, Free q_free) {
-  const ChunkKind kind = rze_decode<false>(sm, sy, m, P, Q, q_free);
-  if (kind != CHUNK_PLANES) return kind;
-  uint32_t w[32];
-  uint32_t before;
-  planes_to_words<false, true>(sm, Q, m.nw, w, before);
-  row_store(Q, threadIdx.x, w);
-  return kind;
 }
 
 }  // namespace cortado

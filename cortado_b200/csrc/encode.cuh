@@ -85,7 +85,7 @@ struct Packer {
 
 // ============================================================== encode stage
 // Input: v[32] = the pre-DIFFMS words of group g = threadIdx.x (quantized bins
-// or residuals; words at or beyond nw are 0) and, for lane 0, the word before
+// or residuals; anything at or beyond m.nw) and, for lane 0, the word before
 // them (prev0, 0 for thread 0).  Y is free on entry; it becomes the plane
 // buffer (d_DIFFMS_4 -> d_BIT_4 -> d_RZE_1, raw fallback).  The payload goes,
 // padded (staged()), to `st`, which may be Y itself and is not written before
@@ -98,18 +98,15 @@ struct Packer {
 // Three hooks run on every thread: planes_written() before the barrier after
 // which the planes are read, planes_ready() after it, and planes_read(n) after
 // the next one, with a bound n of the payload's bytes.
-// FULL: a whole 16 KiB chunk (nw == 4096), with compile-time addressing.
-// KEEP: the plane words stay in registers (st is Y, or a partial chunk); else
-// they are read again for the packing, eight at a time in a loop, which keeps
+// KEEP: the plane words stay in registers (st is Y); else they are read again for the packing, eight at a time in a loop, which keeps
 // the re-encoders' code short.
-template <bool FULL, bool KEEP, typename Written, typename Ready, typename Read>
+template <bool KEEP, typename Written, typename Ready, typename Read>
 __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (&v)[32], uint32_t prev0, uint32_t* Y,
                                              uint32_t* st, uint32_t* st_small, const StageMeta& m, Packer& pz, Packer& pk,
                                              Written planes_written, Ready planes_ready, Read planes_read) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nw = FULL ? CW : m.nw;
+  const int nw = m.nw;
   const int osize = nw * 4;
-  const int G = nw >> 5, rem = nw & 31;
   pz.acc = pk.acc = 0;
 
   // DIFFMS (d_DIFFMS.h:44-66): word minus its predecessor, then zig-zag.
@@ -121,40 +118,33 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
     const uint32_t cur = v[k];
     const uint32_t d = cur - prev;
     prev = cur;
-    v[k] = (FULL || 32 * tid + k < nw) ? (d << 1) ^ (uint32_t)((int32_t)d >> 31) : 0u;
+    v[k] = (d << 1) ^ (uint32_t)((int32_t)d >> 31);
     any |= v[k];
   }
-  // BIT_4: full groups are transposed into the planes (plane s at linear
-  // words s*G .. s*G+G-1); the trailing partial group is copied untransposed.
-  if (FULL) {
-    // the warp's part of plane s is row 4 s + warp of Y
-    const uint32_t bits = __reduce_or_sync(0xffffffffu, any);
-    uint32_t pe, po;
-    plane_offsets(tid, pe, po);
-    int half = 0;
-    if (bits < 0x10000u) {  // planes 0..15 are zero: lanes 2s and 2s + 1 clear row s
-      half = 1;
-      uint4* r = reinterpret_cast<uint4*>(Y + 32 * (4 * (lane >> 1) + warp));
+  // BIT_4: thread g's words are transposed into the planes (plane s at linear
+  // words 128 s ..; the warp's part of it is row 4 s + warp of Y).
+  const uint32_t bits = __reduce_or_sync(0xffffffffu, any);
+  uint32_t pe, po;
+  plane_offsets(tid, pe, po);
+  int half = 0;
+  if (bits < 0x10000u) {  // planes 0..15 are zero: lanes 2s and 2s + 1 clear row s
+    half = 1;
+    uint4* r = reinterpret_cast<uint4*>(Y + 32 * (4 * (lane >> 1) + warp));
 #pragma unroll
-      for (int u = 0; u < 4; u++) r[((lane & 1) << 2 | u) ^ ((lane >> 1) & 7)] = make_uint4(0, 0, 0, 0);
-    }
+    for (int u = 0; u < 4; u++) r[((lane & 1) << 2 | u) ^ ((lane >> 1) & 7)] = make_uint4(0, 0, 0, 0);
+  }
 #pragma unroll 1
-    for (; half < 2; half++) {
-      uint32_t p[16];
+  for (; half < 2; half++) {
+    uint32_t p[16];
 #pragma unroll
-      for (int k = 0; k < 16; k++) p[k] = prmt(v[k], v[k + 16], half ? 0x1054u : 0x3276u);
-      if (bits) transpose_blocks(p);
+    for (int k = 0; k < 16; k++) p[k] = prmt(v[k], v[k + 16], half ? 0x1054u : 0x3276u);
+    if (bits) transpose_blocks(p);
 #pragma unroll
-      for (int s = 0; s < 16; s++) Y[2048 * half + 128 * s + ((s & 1) ? po : pe)] = p[s];
-    }
-  } else if (tid < G) {
-    transpose32(v);
-#pragma unroll
-    for (int s = 0; s < 32; s++) Y[swz(s * G + tid)] = v[s];
-  } else if (tid == G && rem) {
-#pragma unroll
-    for (int k = 0; k < 32; k++)
-      if (k < rem) Y[swz(32 * G + k)] = v[k];
+    for (int s = 0; s < 16; s++) Y[2048 * half + 128 * s + ((s & 1) ? po : pe)] = p[s];
+  }
+  if (nw != CW) {
+    __syncthreads();
+    compact_planes(Y, nw);
   }
   planes_written();
   const bool any_nz = __syncthreads_or(any != 0);
@@ -182,11 +172,6 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
   };
   if (KEEP) {
     row_load(Y, tid, q);
-    if (!FULL && 32 * tid + 32 > nw) {
-#pragma unroll
-      for (int k = 0; k < 32; k++)
-        if (32 * tid + k >= nw) q[k] = 0;
-    }
     uint32_t qany = 0;
 #pragma unroll
     for (int k = 0; k < 32; k++) qany |= q[k];
@@ -211,8 +196,8 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
   uint32_t pb = 0;
   if (tid > 0) {
     const int w = 32 * tid - 2;
-    const uint32_t x0 = (FULL || w < nw) ? Y[swz(w)] : 0u;
-    const uint32_t x1 = (FULL || w + 1 < nw) ? Y[swz(w + 1)] : 0u;
+    const uint32_t x0 = Y[swz(w)];
+    const uint32_t x1 = Y[swz(w + 1)];
     pb = nz_nibble(x0) | (nz_nibble(x1) << 4);
   }
   // Repetition elimination, level 1 (d_REencode4wordsperthread): keep bitmap
@@ -356,23 +341,6 @@ __device__ __forceinline__ void flush_staged(const Ctl& sm, const uint32_t* st, 
     table_out[p.c] = (uint16_t)p.csize;
     if (p.c == chunks - 1) *out_size = HDR + 2 * chunks + (long long)(X + p.csize);
   }
-}
-
-// The partial last chunk of a stream, out of line (it passes its words through
-// the calling thread's own row of Y, never through a pointer to the caller's
-// register array, which would put that array in local memory).  The runs are
-// finished on return; returns whether the chunk is stored raw.
-__device__ __noinline__ bool encode_partial(Ctl& sm, const Sync& sy, uint32_t prev0, uint32_t* Y, uint32_t* st,
-                                            uint32_t* st_small, const StageMeta& m) {
-  uint32_t w[32];
-  row_load(Y, threadIdx.x, w);
-  __syncthreads();  // Y becomes the plane buffer
-  Packer pz(0), pk(0);
-  const bool raw = encode_chunk<false, true>(sm, sy, w, prev0, Y, st, st_small, m, pz, pk, NoHook{}, NoHook{}, [](uint32_t) {});
-  __syncthreads();
-  pz.finish(st);
-  pk.finish(st);
-  return raw;
 }
 
 }  // namespace cortado

@@ -212,55 +212,99 @@ __device__ __forceinline__ void rot_nibbles(const uint32_t (&M)[4], int r, uint3
   R[3] = __funnelshift_r(a3, a0, bs);
 }
 
+// The partial last chunk of a stream (nw < 4096 words, G whole groups and a
+// remainder that BIT_4 copies untransposed) runs through the full chunks' code:
+// these two move its BIT_4 output (plane s at words s*G .. s*G+G-1, then the
+// remainder) to and from the full chunk's place in a plane buffer (plane s at
+// words 128*s ..), padded with zeros.  Eight planes move per step, in the order
+// in which no step writes over a later one's source; warp 0 transposes the
+// remainder with one vote per plane or word.  Out of line and short: small
+// launches mostly wait for instructions to be fetched, and a partial chunk ends
+// them (a second copy of the stages for partial chunks took 4 us more).
+// Called by every thread; ends with a barrier, expects one before.
+__device__ __noinline__ void widen_planes(uint32_t* Y, int nw) {
+  const int tid = threadIdx.x, lane = tid & 31, G = nw >> 5, rem = nw & 31;
+  uint32_t z = (tid < rem) ? Y[swz(32 * G + tid)] : 0u, mine = 0;
+  if (tid < 32) {
+    for (int s = 0; s < 32; s++) {
+      const uint32_t p = __brev(__ballot_sync(0xffffffffu, (z >> (31 - s)) & 1u));
+      if (lane == s) mine = p;  // plane s of the remainder
+    }
+  }
+#pragma unroll 1
+  for (int s0 = 24; s0 >= 0; s0 -= 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = tid < G ? Y[swz((s0 + i) * G + tid)] : 0u;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; i++) Y[swz(128 * (s0 + i) + tid)] = v[i];
+    __syncthreads();
+  }
+  if (tid < 32) Y[swz(128 * tid + G)] = mine;
+  __syncthreads();
+}
+__device__ __noinline__ void compact_planes(uint32_t* Y, int nw) {
+  const int tid = threadIdx.x, lane = tid & 31, G = nw >> 5, rem = nw & 31;
+  uint32_t p = tid < 32 ? Y[swz(128 * tid + G)] : 0u, mine = 0;
+  if (tid < 32) {
+    for (int k = 0; k < rem; k++) {
+      const uint32_t z = __brev(__ballot_sync(0xffffffffu, (p >> (31 - k)) & 1u));
+      if (lane == k) mine = z;  // word k of the remainder
+    }
+  }
+#pragma unroll 1
+  for (int s0 = 0; s0 < 32; s0 += 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = Y[swz(128 * (s0 + i) + tid)];
+    __syncthreads();
+    if (tid < G) {
+#pragma unroll
+      for (int i = 0; i < 8; i++) Y[swz((s0 + i) * G + tid)] = v[i];
+    }
+    __syncthreads();
+  }
+  for (int w = 32 * G + tid; w < CW; w += NT) Y[swz(w)] = w < nw ? mine : 0u;  // (tid < rem in warp 0 holds word tid)
+  __syncthreads();
+}
+
 // Inverse of DIFFMS + BIT_4 for a chunk whose BIT_4 output sits in the
 // swizzled plane buffer: gathers the plane words of group g = threadIdx.x,
 // transposes them back, undoes the zig-zag and the differences (in-thread
 // prefix sum plus a block scan of the group totals), and returns the group's
-// words in v[32] (words at or beyond nw are 0) and the word before them in
-// `before` (0 for the first group).  Ends with a barrier (the scan's), after
-// which the plane buffer may be reused.  SHORT: loops are not unrolled (the
-// re-encoders, whose code is long).
-template <bool FULL, bool SHORT>
-__device__ __forceinline__ void planes_to_words(Ctl& sm, const uint32_t* plane, int nw_in, uint32_t (&v)[32],
-                                                uint32_t& before) {
+// words in v[32] and the word before them in `before` (0 for the first group).
+// (Words behind a partial chunk's end repeat its last one.)  Ends with a
+// barrier (the scan's), after which the plane buffer may be reused.  SHORT:
+// loops are not unrolled (the re-encoders, whose code is long).
+template <bool SHORT>
+__device__ __forceinline__ void planes_to_words(Ctl& sm, const uint32_t* plane, uint32_t (&v)[32], uint32_t& before) {
   const int tid = threadIdx.x;
-  const int nw = FULL ? CW : nw_in;
-  const int G = nw >> 5, rem = nw & 31;
   // ---- undo BIT_4 (d_iBIT_4): gather plane words of group g, transpose.
-  bool live = true;
-  if (FULL) {
-    uint32_t pe, po;
-    plane_offsets(tid, pe, po);
-    uint32_t h[16], p[16];  // planes 0..15 and 16..31, transposed
+  uint32_t pe, po;
+  plane_offsets(tid, pe, po);
+  uint32_t h[16], p[16];  // planes 0..15 and 16..31, transposed
 #pragma unroll
-    for (int s = 0; s < 16; s++) p[s] = 0;
-    live = false;
+  for (int s = 0; s < 16; s++) p[s] = 0;
+  bool live = false;
 #pragma unroll(SHORT ? 1 : 2)
-    for (int half = 0; half < 2; half++) {
-      uint32_t any = 0;
+  for (int half = 0; half < 2; half++) {
+    uint32_t any = 0;
 #pragma unroll
-      for (int s = 0; s < 16; s++) {
-        h[s] = p[s];
-        p[s] = plane[2048 * half + 128 * s + ((s & 1) ? po : pe)];
-        any |= p[s];
-      }
-      if (__any_sync(0xffffffffu, any != 0)) {
-        transpose_blocks(p);
-        live = true;
-      }
+    for (int s = 0; s < 16; s++) {
+      h[s] = p[s];
+      p[s] = plane[2048 * half + 128 * s + ((s & 1) ? po : pe)];
+      any |= p[s];
     }
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-      v[k] = __byte_perm(p[k], h[k], 0x7632);
-      v[k + 16] = __byte_perm(p[k], h[k], 0x5410);
+    if (__any_sync(0xffffffffu, any != 0)) {
+      transpose_blocks(p);
+      live = true;
     }
-  } else if (tid < G) {
+  }
 #pragma unroll
-    for (int s = 0; s < 32; s++) v[s] = plane[swz(s * G + tid)];
-    transpose32(v);
-  } else {
-#pragma unroll
-    for (int k = 0; k < 32; k++) v[k] = (tid == G && k < rem) ? plane[swz(32 * G + k)] : 0u;
+  for (int k = 0; k < 16; k++) {
+    v[k] = __byte_perm(p[k], h[k], 0x7632);
+    v[k + 16] = __byte_perm(p[k], h[k], 0x5410);
   }
   // ---- undo DIFFMS (d_iDIFFMS, d_DIFFMS.h:69-102): un-zig-zag, prefix sum.
   uint32_t acc = 0;
@@ -272,16 +316,11 @@ __device__ __forceinline__ void planes_to_words(Ctl& sm, const uint32_t* plane, 
       v[k] = acc;
     }
   }
-  uint32_t dummy;
-  const uint32_t carry = block_scan_excl(acc, sm.scan_c, dummy);  // (its barrier: every plane read is done)
+  uint32_t total;
+  const uint32_t carry = block_scan_excl(acc, sm.scan_c, total);  // (its barrier: every plane read is done)
 #pragma unroll
   for (int k = 0; k < 32; k++) v[k] += carry;
   before = carry;
-  if (!FULL && 32 * tid + 32 > nw) {
-#pragma unroll
-    for (int k = 0; k < 32; k++)
-      if (32 * tid + k >= nw) v[k] = 0;
-  }
 }
 
 }  // namespace cortado
