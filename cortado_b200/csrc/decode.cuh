@@ -72,6 +72,14 @@ __device__ __forceinline__ void re_expand8(const uint32_t* P, int pos, bool firs
 }
 
 // ---------------------------------------------------------------- RZE decode
+// Chunks of at most this many zero-eliminated bytes are expanded word by
+// non-zero word.
+constexpr uint32_t FEW = 512;
+constexpr uint32_t QFEW = 4;  // the same for a quarter of a segment
+// Where a segment's masks and byte positions (8 words) are handed over: its own
+// row of the plane buffer, at a place that spreads over the banks.
+__device__ __forceinline__ uint32_t* seg_info(uint32_t* Q, int seg) { return Q + 32 * seg + 8 * (seg & 3); }
+
 enum ChunkKind : int { CHUNK_ZERO = 0, CHUNK_PLANES = 1, CHUNK_RAW = 2 };
 
 // Undoes RZE_1 (d_iRZE, d_RZE.h:127-206) for the chunk whose payload the
@@ -177,15 +185,15 @@ __device__ __forceinline__ ChunkKind rze_decode(Ctl& sm, const Sync& sy, const S
     latch(sy.status, DST_CORRUPT);
     M[0] = M[1] = M[2] = M[3] = 0;
   }
-  // ZE decode: scatter the non-zero bytes back into the 32 words.
-  uint32_t* row = Q + 32 * tid;
-  const uint32_t xr = tid & 7u;
-  uint32_t p = (uint32_t)d + zoff;
-  if (__reduce_max_sync(0xffffffffu, nz) <= 12) {
-    // few bytes: zero rows, then the non-zero words
+  // ZE decode: scatter the non-zero bytes back into the words.
+  if (NZ <= FEW) {
+    // few bytes: every thread clears its segment and fills in the non-zero words
+    uint32_t* row = Q + 32 * tid;
+    const uint32_t xr = tid & 7u;
     uint4* r4 = reinterpret_cast<uint4*>(row);
 #pragma unroll
     for (int u = 0; u < 8; u++) r4[u ^ xr] = make_uint4(0, 0, 0, 0);
+    uint32_t p = (uint32_t)d + zoff;
 #pragma unroll
     for (int part = 0; part < 4; part++) {
       uint32_t m32 = M[part];
@@ -201,38 +209,62 @@ __device__ __forceinline__ ChunkKind rze_decode(Ctl& sm, const Sync& sy, const S
       }
     }
   } else {
-    // Every word, two at a time, each lane starting at another pair (lane / 2):
-    // lanes' bytes are up to 128 bytes apart, and in the same order their
-    // reads would fall into the same banks.  R: the mask rotated to that start.
-    // (A loop over four words of the mask: unrolled whole, it made every kernel
-    // slower on dense data, init_recv of 256 MiB at 25% 157 -> 164 us, and the
-    // re-encoders stall on instruction fetch.)
-    const uint32_t rot = ((uint32_t)lane >> 1) * 2;
-    uint32_t R[4];
-    rot_nibbles(M, rot, R);
-    p += rot ? nibble_prefix(M, rot) : nz;
-    uint32_t k = rot;
+    // The non-zero bytes of real data lie in the low planes, the last segments.
+    // So that all warps share them, the segments are expanded 32 at a time, a
+    // quarter of one (8 words) per thread; a segment's masks and byte positions
+    // pass through its own row of Q.  (With a segment per thread one or two
+    // warps did all the work while the others waited at the barrier: 256 MiB,
+    // init_recv 137 -> 133 us at 6% of the size, resi_send 310 -> 303 us.  The
+    // same split of the encoders' packing cost as much as it gave.)
+    {
+      uint4* info = reinterpret_cast<uint4*>(seg_info(Q, tid));
+      info[0] = make_uint4(M[0], M[1], M[2], M[3]);
+      const uint32_t p0 = (uint32_t)d + zoff, p1 = p0 + __popc(M[0]), p2 = p1 + __popc(M[1]);
+      info[1] = make_uint4(p0, p1, p2, p2 + __popc(M[2]));
+    }
+    __syncthreads();
+    const uint32_t quarter = tid & 3, rot = (tid >> 2) & 3;  // quarters start at different words (banks)
 #pragma unroll 1
-    for (int i = 0; i < 4; i++) {
-      const uint32_t r = R[0];
-      R[0] = R[1];
-      R[1] = R[2];
-      R[2] = R[3];
+    for (int seg = tid >> 2; seg < NT; seg += 32) {
+      const uint32_t* info = seg_info(Q, seg) + quarter;
+      uint32_t m = info[0], p = info[4];
+      uint32_t* row = Q + 32 * seg;
+      const uint32_t x = ((seg & 7) << 2) ^ (8 * quarter);  // word k of the quarter: row[k ^ x]
+      const uint32_t n = __popc(m);
+      if (__any_sync(0xffffffffu, n > QFEW)) {  // (also: the warp has read its segments' masks)
+        const uint32_t R = __funnelshift_r(m, m, 8 * rot);
+        p += rot ? __popc(m & ((1u << (8 * rot)) - 1u)) : n;
+        uint32_t k = 2 * rot;
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        if (k == 0) p -= nz;  // back to the first word's bytes
-        const uint32_t mk = prmt(r, 0u, 0x4440u | j);
-        uint32_t s0, s1;
-        spread_sel2(mk, s0, s1);
-        const uint32_t* w = reinterpret_cast<const uint32_t*>(st + (p & ~3u));
-        uint2 q;
-        q.x = prmt(__funnelshift_r(w[0], w[1], 8 * p), 0u, s0);
-        p += __popc(mk & 15u);
-        w = reinterpret_cast<const uint32_t*>(st + (p & ~3u));
-        q.y = prmt(__funnelshift_r(w[0], w[1], 8 * p), 0u, s1);
-        p += __popc(mk >> 4);
-        *reinterpret_cast<uint2*>(row + (k ^ (xr << 2))) = q;
-        k = (k + 2) & 30u;
+        for (int j = 0; j < 4; j++) {
+          if (k == 0) p -= n;  // back to the quarter's first bytes
+          const uint32_t mk = prmt(R, 0u, 0x4440u | j);
+          uint32_t s0, s1;
+          spread_sel2(mk, s0, s1);
+          const uint32_t* w = reinterpret_cast<const uint32_t*>(st + (p & ~3u));
+          uint2 q;
+          q.x = prmt(__funnelshift_r(w[0], w[1], 8 * p), 0u, s0);
+          p += __popc(mk & 15u);
+          w = reinterpret_cast<const uint32_t*>(st + (p & ~3u));
+          q.y = prmt(__funnelshift_r(w[0], w[1], 8 * p), 0u, s1);
+          p += __popc(mk >> 4);
+          *reinterpret_cast<uint2*>(row + (k ^ x)) = q;
+          k = (k + 2) & 6u;
+        }
+      } else {  // few bytes: clear the quarter, fill in the non-zero words
+        uint4* r4 = reinterpret_cast<uint4*>(row);
+        r4[(2 * quarter) ^ (seg & 7)] = make_uint4(0, 0, 0, 0);
+        r4[(2 * quarter + 1) ^ (seg & 7)] = make_uint4(0, 0, 0, 0);
+        while (m) {
+          const uint32_t b = (__ffs(m) - 1) & 28u;
+          const uint32_t mk = (m >> b) & 15u;
+          m ^= mk << b;
+          const uint32_t* w = reinterpret_cast<const uint32_t*>(st + (p & ~3u));
+          uint32_t s0, s1;
+          spread_sel2(mk, s0, s1);
+          row[(b >> 2) ^ x] = prmt(__funnelshift_r(w[0], w[1], 8 * p), 0u, s0);
+          p += __popc(mk);
+        }
       }
     }
   }
