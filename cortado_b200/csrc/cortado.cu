@@ -49,18 +49,33 @@ __device__ __forceinline__ Ctl& ctl_block() {
 // buffer after a TMA store must be the one that issued the store.
 constexpr int TMA_TID = 96;
 
-// Reads this launch's lookback epoch and sets up the stage barriers (every
-// CTA, at start; the caller synchronizes).  A stage's barrier completes a
-// phase per use: two arrivals by the prefetching lane (one before its loads
-// are issued, one after the stage's metadata and hand-copied bytes are
-// written) plus the TMA bytes, so waiting on it also publishes the metadata.
-__device__ __forceinline__ void begin_launch(Ctl& sm, const Sync& sy) {
-  if (threadIdx.x == 0) sm.epoch = *(volatile unsigned int*)sy.epoch;
+// Start of every CTA: takes its place in the launch's queue, reads the lookback
+// epoch (both reads in flight together) and sets up the barriers.  The queue
+// hands out the helper's place first (when there are at least two CTAs), then
+// the chunks in order: a CTA's first place is also its first chunk, and every
+// chunk handed out belongs to a CTA that is running.  Returns whether this CTA
+// is the helper.  A chunk's barrier completes a phase per use: two arrivals by
+// the prefetching lane (one before its loads are issued, one after the chunk's
+// metadata and hand-copied bytes are written) plus the TMA bytes, so waiting on
+// it also publishes the metadata.
+__device__ __forceinline__ unsigned int next_place(const Sync& sy) {
+  return atomicAdd(&sy.counter[0], 1u) - (gridDim.x < 2 ? 0u : 1u);
+}
+__device__ __forceinline__ bool begin_launch(Ctl& sm, const Sync& sy) {
+  if (threadIdx.x == 0) {
+    const unsigned int e = *(volatile unsigned int*)sy.epoch;
+    const unsigned int p = next_place(sy);
+    sm.epoch = e;
+    sm.first = p;
+    sm.pend.valid = 0;
+  }
   if (threadIdx.x == TMA_TID) {
     mbar_init(&sm.bar, 2);
     mbar_init(&sm.bar_src, 1);
     fence_mbar_init();
   }
+  __syncthreads();
+  return sm.first == 0xffffffffu;
 }
 
 // The last CTA out resets the chunk queue and advances the epoch for the next
@@ -88,7 +103,6 @@ __device__ __forceinline__ unsigned int finish_launch(Ctl& sm, const Sync& sy, b
       *sy.epoch = (e == 65535u) ? 0u : e + 1u;
       sy.counter[0] = 0;
       sy.counter[1] = 0;
-      sy.counter[6] = 0;
       __threadfence();
     }
   }
@@ -337,17 +351,14 @@ template <class Src>
 __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& sy) {
   constexpr int LOADER = 1;  // the warp that takes chunks: its planes are rarely the dense ones
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  begin_launch(sm, sy);
-  init_pack_table();
-  if (tid == 0) sm.pend.valid = 0;
+  init_pack_table();  // (read after the loop's first barrier)
   WalkState ws{-1};
-  __syncthreads();
-  auto take = [&]() -> unsigned int { return (warp == LOADER && lane == 0) ? atomicAdd(&sy.counter[0], 1u) : 0u; };
+  auto take = [&]() -> unsigned int { return (warp == LOADER && lane == 0) ? next_place(sy) : 0u; };
   auto load = [&](int t, unsigned int g) {
     if (warp == LOADER) prefetch_floats(sm, t, __shfl_sync(0xffffffffu, g, 0), src, ws);
   };
   auto flush = [&](int t) { write_pending<true>(sm, src, stage_buf(sm, t), stage_buf(sm, t) + CW); };
-  load(0, take());
+  load(0, sm.first);
   int s = 0;  // this chunk's buffer and slots; also the barrier's phase
   for (;; s ^= 1) {
     if (!mbar_wait(&sm.bar, s, sy.timeout_ns)) latch(sy.status, DST_TIMEOUT);
@@ -401,10 +412,9 @@ __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& 
   flush(s ^ 1);
 }
 
-// ---- stream prefetch (warp FEEDER of a decoder or re-encoder CTA), in two
-// parts.  The payload offset comes from the launch's offset scanner (the prefix
-// sum of the size table that the reference's decoders form per CTA,
-// d_s2c.h:98-106).
+// ---- stream prefetch (one warp of a decoder or re-encoder CTA), in two parts.
+// The payload offset comes from the launch's offset scanner (the prefix sum of
+// the size table that the reference's decoders form per CTA, d_s2c.h:98-106).
 constexpr int FEEDER = TMA_TID / 32;
 
 // What resolve_stream leaves in flight (lane 0), until park_stream puts it into
@@ -477,6 +487,10 @@ __device__ __forceinline__ void park_stream(Ctl& sm, int t, const Src& src, cons
   __syncwarp();
 }
 
+// Chunks below this one sum the sizes before them themselves when the scanner
+// has not published their offset yet: at most eight loads per lane.
+constexpr int OWN_SUM = 256;
+
 // Second part, once the place at byte `at` (a multiple of 16) of P is free: the
 // payload's 16-byte-aligned span with one bulk copy, the ragged tail by the
 // lanes.
@@ -495,12 +509,19 @@ __device__ __forceinline__ void issue_stream(Ctl& sm, int t, const Src& src, uin
     return;
   }
   const OpArgs& A = src.args(m.item);
-  unsigned long long off = 0;
-  if (lane == 0) {
-    const unsigned long long w = m.off;
-    off = ((w >> 48) == sm.epoch && (w & LB_INC)) ? w & LB_VAL : wait_offset(A.sy, sm.epoch, m.c);
+  unsigned long long off = m.off;
+  if ((off >> 48) == sm.epoch && (off & LB_INC)) {
+    off &= LB_VAL;
+  } else if (m.c < OWN_SUM) {
+    // (the scanner is still starting: a small launch would wait for it)
+    unsigned int sum = 0;
+    const uint16_t* table = reinterpret_cast<const uint16_t*>(A.in + HDR);
+    for (int i = lane; i < (int)m.c; i += 32) sum += table[i];
+    off = __reduce_add_sync(0xffffffffu, sum);
+  } else {
+    if (lane == 0) off = wait_offset(A.sy, sm.epoch, m.c);
+    off = __shfl_sync(0xffffffffu, off, 0);
   }
-  off = __shfl_sync(0xffffffffu, off, 0);
   const int cs = m.csize;
   __syncwarp();  // (lane 0 rewrites it below)
   const int osize = 4 * m.nw;
@@ -703,18 +724,17 @@ __device__ __forceinline__ int room_out(int n) { return n + (n >> 5) + 32; }
 template <int OP, bool APPLY, class Src>
 __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Sync& sy) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  begin_launch(sm, sy);
-  init_pack_table();
-  if (tid == 0) sm.pend.valid = 0;
-  __syncthreads();  // sm.epoch
-  if (gridDim.x == 1 && warp == 1) src.scan(sm.epoch);
-  __syncthreads();
+  init_pack_table();  // (read after the loop's first barrier)
+  if (gridDim.x == 1) {
+    if (warp == 1) src.scan(sm.epoch);
+    __syncthreads();
+  }
   uint32_t* Y = stage_buf(sm, 0);
   uint32_t* R = Y + CW;
-  const bool feeder = warp == FEEDER;
+  const bool feeder = warp == 1;  // (warp 3 packs the densest planes: 1% slower)
   WalkState ws{-1};
   Ahead ah{0, 0};
-  auto take = [&]() -> unsigned int { return (feeder && lane == 0) ? atomicAdd(&sy.counter[0], 1u) : 0u; };
+  auto take = [&]() -> unsigned int { return (feeder && lane == 0) ? next_place(sy) : 0u; };
   auto resolve = [&](int t, unsigned int g) {
     if (feeder) resolve_stream<OP>(sm, t, __shfl_sync(0xffffffffu, g, 0), src, ws, ah);
   };
@@ -724,7 +744,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
   auto issue = [&](int t) {  // (feeder)
     issue_stream(sm, t, src, reinterpret_cast<uint8_t*>(R), ROOM - room_in(min(sm.st[t].csize, CS)));
   };
-  resolve(0, take());
+  resolve(0, sm.first);
   park(0);
   if (feeder) issue(0);
   for (int s = 0;; s ^= 1) {  // s: the metadata slot, and the barrier's phase
@@ -843,10 +863,10 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
 template <int OP, class Src>
 __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync& sy) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  begin_launch(sm, sy);
-  __syncthreads();
-  if (gridDim.x == 1 && warp == 1) src.scan(sm.epoch);
-  __syncthreads();
+  if (gridDim.x == 1) {
+    if (warp == 1) src.scan(sm.epoch);
+    __syncthreads();
+  }
   uint32_t* P = stage_buf(sm, 0);
   uint32_t* Q = stage_buf(sm, 1);
   const bool feeder = warp == FEEDER;
@@ -854,10 +874,8 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
   Ahead ah{0, 0};
   long long pending = 0;
   if (feeder) {
-    long long g0 = 0;
-    if (lane == 0) g0 = atomicAdd(&sy.counter[0], 1u);
-    resolve_stream<OP>(sm, 0, __shfl_sync(0xffffffffu, g0, 0), src, ws, ah);
-    if (lane == 0) pending = atomicAdd(&sy.counter[0], 1u);
+    resolve_stream<OP>(sm, 0, sm.first, src, ws, ah);
+    if (lane == 0) pending = next_place(sy);
     park_stream(sm, 0, src, ah);
     issue_stream(sm, 0, src, reinterpret_cast<uint8_t*>(P), 0);
   }
@@ -870,7 +888,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     if (feeder) {
       // (every other thread is past the previous chunk's last use of this slot)
       const long long gp = __shfl_sync(0xffffffffu, pending, 0);
-      if (lane == 0) pending = atomicAdd(&sy.counter[0], 1u);
+      if (lane == 0) pending = next_place(sy);
       resolve_stream<OP>(sm, s ^ 1, gp, src, ws, ah);
     }
     const int item = m.item;
@@ -1008,19 +1026,8 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
 // when other kernels share the GPU and not every CTA of the launch fits at
 // once, so the CTAs that wait for its offsets cannot wait for a CTA that
 // waits for them.  A one-CTA launch scans its offsets itself first.
-__device__ __forceinline__ bool helper_cta(Ctl& sm, const Sync& sy) {
-  if (gridDim.x < 2) return false;
-  if (threadIdx.x == 0) sm.is_last = atomicAdd(&sy.counter[6], 1u) == 0;
-  __syncthreads();
-  const bool h = sm.is_last;
-  __syncthreads();
-  return h;
-}
-
 template <bool RESOLVE, bool SCAN, class Src>
 __device__ __forceinline__ void run_helper(Ctl& sm, const Src& src, const Sync& sy) {
-  begin_launch(sm, sy);
-  __syncthreads();
   const int warp = threadIdx.x >> 5;
   if (RESOLVE && sy.resolver && warp == 0) resolve_loop(sy, sm.epoch, src.total);
   if (SCAN && warp == 1) src.scan(sm.epoch);
@@ -1041,7 +1048,7 @@ __global__ void __launch_bounds__(NT, MINB_STORE) k_store(const __grid_constant_
     }
   }
   const SingleSrc src{&a, &map_in, nullptr, chunks, StreamHdr{}, q1, q2};
-  if (helper_cta(sm, a.sy)) run_helper<true, false>(sm, src, a.sy);
+  if (begin_launch(sm, a.sy)) run_helper<true, false>(sm, src, a.sy);
   else store_loop(sm, src, a.sy);
   finish_launch(sm, a.sy);
 }
@@ -1065,7 +1072,7 @@ __global__ void __launch_bounds__(NT, MINB_REENC) k_reencode(const __grid_consta
     }
   }
   const SingleSrc src{&a, nullptr, nullptr, h.chunks, h, q1, q2};
-  if (helper_cta(sm, a.sy)) run_helper<true, true>(sm, src, a.sy);
+  if (begin_launch(sm, a.sy)) run_helper<true, true>(sm, src, a.sy);
   else reencode_loop<OP, APPLY>(sm, src, a.sy);
   finish_launch(sm, a.sy);
 }
@@ -1083,7 +1090,7 @@ __global__ void __launch_bounds__(NT, OP == OP_RAPPLY ? MINB_RAPPLY : MINB_DEC) 
     *a.out_size = hdr_ok ? h.n : 0;
   }
   const SingleSrc src{&a, &map_src, &map_out, h.chunks, h, a.q1, a.q2};
-  if (helper_cta(sm, a.sy)) run_helper<false, true>(sm, src, a.sy);
+  if (begin_launch(sm, a.sy)) run_helper<false, true>(sm, src, a.sy);
   else decode_loop<OP>(sm, src, a.sy);
   finish_launch(sm, a.sy);
 }
@@ -1095,7 +1102,7 @@ k_batch(const BatchItem* __restrict__ items, int n_items, long long total_chunks
   Ctl& sm = ctl_block();
   const BatchSrc<OP> src{items, n_items, total_chunks};
   constexpr bool encoder = OP == OP_STORE || OP == OP_S2C || OP == OP_RESI;
-  if (helper_cta(sm, sy)) run_helper<encoder, OP != OP_STORE>(sm, src, sy);
+  if (begin_launch(sm, sy)) run_helper<encoder, OP != OP_STORE>(sm, src, sy);
   else if (OP == OP_STORE) store_loop(sm, src, sy);
   else if (encoder) reencode_loop<OP, APPLY>(sm, src, sy);
   else decode_loop<OP>(sm, src, sy);
@@ -1105,8 +1112,8 @@ k_batch(const BatchItem* __restrict__ items, int n_items, long long total_chunks
 // ---- store without allocation (cortado_store_encode_noalloc)
 // Fixed scratch for callers that cannot allocate device memory: one
 // lookback word per chunk for up to CORTADO_NOALLOC_MAX_BYTES of input, then
-// the chunk queue, the finished-CTA count, the status word, the epoch and the
-// helper ticket (32-bit words 0, 1, 2, 3 and 6 of the last 4 entries).  Every GPU that
+// the chunk queue, the finished-CTA count, the status word and the epoch
+// (32-bit words 0, 1, 2 and 3 of the last 4 entries).  Every GPU that
 // loads the library holds this array until the process exits.
 constexpr long long NOALLOC_CHUNKS = CORTADO_NOALLOC_MAX_BYTES / CS;
 __device__ __align__(256) unsigned long long g_noalloc_scratch[NOALLOC_CHUNKS + 4];
@@ -1123,7 +1130,7 @@ __global__ void __launch_bounds__(NT, MINB_STORE) k_store_noalloc(const __grid_c
     if (chunks == 0) *a.out_size = HDR;
   }
   const SingleSrc src{&a, &map_in, nullptr, chunks, StreamHdr{}, a.q1, a.q2};
-  if (helper_cta(sm, a.sy)) run_helper<true, false>(sm, src, a.sy);
+  if (begin_launch(sm, a.sy)) run_helper<true, false>(sm, src, a.sy);
   else store_loop(sm, src, a.sy);
   const unsigned int st = finish_launch(sm, a.sy, true);
   if (st) *a.out_size = -(long long)st;
@@ -1278,7 +1285,7 @@ struct cortado_ctx {
   int grid_store = 0, grid_reenc = 0, grid_dec = 0, grid_rapply = 0;
   unsigned long long* flags = nullptr;
   long long flags_cap = 0;
-  unsigned int* words = nullptr;  // [0] queue, [1] finished, [2] status, [3..4] minmax, [5] epoch, [6] helper ticket, [7] range blocks finished
+  unsigned int* words = nullptr;  // [0] queue, [1] finished, [2] status, [3..4] minmax, [5] epoch, [7] range blocks finished
   int grid_batch[6] = {0, 0, 0, 0, 0, 0};
   int ctas_override[6] = {0, 0, 0, 0, 0, 0};  // per op: resident CTAs per SM (0 = occupancy limit)
   int resolver[6] = {1, 1, 1, 1, 1, 1};        // per op: lookback resolver warp on (encoders)

@@ -58,7 +58,7 @@ struct Sync {
   unsigned long long* flags;  // lookback words, one per chunk (encoders)
   unsigned long long* offs;   // input payload offsets, one per chunk (decoders, re-encoders), or null
   long long flags_cap;        // words in flags and in offs (cleared when the epoch wraps)
-  unsigned int* counter;      // [0] chunk queue, [1] CTAs finished, [6] helper ticket
+  unsigned int* counter;      // [0] queue of the helper's place and the chunks, [1] CTAs finished
   unsigned int* status;       // first error latched
   unsigned int* epoch;        // 0..65535, tags this launch's lookback words
   unsigned long long timeout_ns;

@@ -113,6 +113,7 @@ struct __align__(16) Ctl {
   Pend pend;                // encoders: the chunk whose payload waits to be flushed
   unsigned long long payload_off;
   unsigned int epoch, is_last;
+  unsigned int first;       // the CTA's first place in the queue (all ones: the helper)
   unsigned int held;        // re-encoders: the next payload waits for room
   unsigned int src_side;    // resi_recv: this chunk's client floats are behind the next payload
 };
