@@ -67,7 +67,7 @@ __device__ __forceinline__ bool begin_launch(Ctl& sm, const Sync& sy) {
     const unsigned int p = next_place(sy);
     sm.epoch = e;
     sm.first = p;
-    sm.pend.valid = 0;
+    sm.pend[0].valid = sm.pend[1].valid = 0;
   }
   if (threadIdx.x == TMA_TID) {
     mbar_init(&sm.bar, 2);
@@ -319,34 +319,37 @@ __device__ __noinline__ uint32_t requant_words(uint32_t* buf, uint32_t m, uint32
   return slow_before ? requant(before) : before;
 }
 
-// Resolves the pending chunk's output offset (warp 0, before a barrier that
+// Resolves a pending chunk's output offset (one warp, before a barrier that
 // publishes sm.payload_off) ...
 template <class Src>
-__device__ __forceinline__ void resolve_pending(Ctl& sm, const Src& src) {
-  const Pend& pd = sm.pend;
-  if (threadIdx.x < 32 && pd.valid) {
+__device__ __forceinline__ void resolve_pending(Ctl& sm, const Src& src, const Pend& pd, int by = 0) {
+  if ((threadIdx.x >> 5) == by && pd.valid) {
     const unsigned long long X = lookback_resolve(src.args(pd.item).sy, sm.epoch, pd.c, pd.csize);
-    if (threadIdx.x == 0) sm.payload_off = X;
+    if ((threadIdx.x & 31) == 0) sm.payload_off = X;
   }
 }
 // ... and writes it out from its staging buffer (every thread, after that
 // barrier).
 // FLOATS: a raw chunk's payload is the input's floats, read again.
 template <bool FLOATS, class Src>
-__device__ __forceinline__ void write_pending(Ctl& sm, const Src& src, const uint32_t* st, const uint32_t* st_small) {
-  const Pend& pd = sm.pend;
+__device__ __forceinline__ void write_pending(Ctl& sm, const Src& src, const Pend& pd, const uint32_t* st,
+                                              const uint32_t* st_small) {
   if (!pd.valid) return;
   const OpArgs& Q = src.args(pd.item);
   const long long chunks = (Q.n + CS - 1) / CS;
-  flush_staged(sm, st, st_small, FLOATS ? reinterpret_cast<const uint32_t*>(Q.in) + pd.c * (long long)CW : nullptr,
+  flush_staged(sm, pd, st, st_small, FLOATS ? reinterpret_cast<const uint32_t*>(Q.in) + pd.c * (long long)CW : nullptr,
                Q.out + HDR + 2 * chunks, reinterpret_cast<uint16_t*>(Q.out + HDR), Q.out_size, chunks);
 }
 
 // store (d_server_encode_kernel): floats -> SQ -> encode.  One buffer (A)
 // receives a chunk's floats, which are quantized into registers, and then
 // takes its planes and its payload; the other (B) holds the previous chunk's
-// payload until it is flushed, while the planes are read, and receives the next
-// chunk after that.
+// payload until it is flushed, and receives the next chunk after that.
+// The previous chunk's offset is waited for only after this chunk's size has
+// been published.  (Waiting before that, although the flush then hid the next
+// load, let one late chunk hold up every CTA's next size: the wait took 3,000
+// to 5,500 of 13,000 to 20,000 cycles per chunk.  256 MiB: nearly all zero bins
+// 156 -> 137 us, sinusoids with noise 166 -> 160, dense 217 -> 214.)
 template <class Src>
 __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& sy) {
   constexpr int LOADER = 1;  // the warp that takes chunks: its planes are rarely the dense ones
@@ -357,7 +360,7 @@ __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& 
   auto load = [&](int t, unsigned int g) {
     if (warp == LOADER) prefetch_floats(sm, t, __shfl_sync(0xffffffffu, g, 0), src, ws);
   };
-  auto flush = [&](int t) { write_pending<true>(sm, src, stage_buf(sm, t), stage_buf(sm, t) + CW); };
+  auto flush = [&](int t) { write_pending<true>(sm, src, sm.pend[t], stage_buf(sm, t), stage_buf(sm, t) + CW); };
   load(0, sm.first);
   int s = 0;  // this chunk's buffer and slots; also the barrier's phase
   for (;; s ^= 1) {
@@ -397,17 +400,21 @@ __device__ __forceinline__ void store_loop(Ctl& sm, const Src& src, const Sync& 
     unsigned int g = 0;
     Packer pz(0), pk(0);
     encode_chunk<true>(
-        sm, A_.sy, v, prev0, A, A, A + CW, m, pz, pk, [&]() { resolve_pending(sm, src); },
-        [&]() {
-          g = take();
-          flush(s ^ 1);
-        },
-        [&](uint32_t) { load(s ^ 1, g); });
-    __syncthreads();  // the payload's full words are in place
+        sm, A_.sy, v, prev0, A, A, A + CW, m, sm.pend[s], pz, pk, []() {}, [&]() { g = take(); },
+        [&](uint32_t) {
+          // the next chunk's floats are loaded after the flush: bring them into L2
+          if (!Src::batched && warp == LOADER && lane == 0 && (long long)g + 1 < src.total)
+            prefetch_l2(A_.in + (long long)g * CS, CS);
+        });
+    resolve_pending(sm, src, sm.pend[s ^ 1], LOADER);
+    __syncthreads();  // the payload's full words are in place; sm.payload_off
+    flush(s ^ 1);
     pz.finish(A);
     pk.finish(A);
+    __syncthreads();  // the other buffer is free
+    load(s ^ 1, g);
   }
-  resolve_pending(sm, src);
+  resolve_pending(sm, src, sm.pend[s ^ 1]);
   __syncthreads();
   flush(s ^ 1);
 }
@@ -689,11 +696,11 @@ __device__ __noinline__ void raw_rebuild(Ctl& sm, uint32_t* X, int nw, uint32_t*
 template <class Src>
 __device__ __noinline__ void flush_now(Ctl& sm, const Src src, uint32_t* R) {
   __syncthreads();
-  resolve_pending(sm, src);
+  resolve_pending(sm, src, sm.pend[0]);
   __syncthreads();
-  write_pending<false>(sm, src, R, R);
+  write_pending<false>(sm, src, sm.pend[0], R, R);
   __syncthreads();
-  if (threadIdx.x == 0) sm.pend.valid = 0;
+  if (threadIdx.x == 0) sm.pend[0].valid = 0;
 }
 
 // init_send / resi_send (d_s2c_encode_kernel, d_residual_encode_kernel):
@@ -823,12 +830,12 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
     __syncthreads();  // the rows of Y are free
     Packer pz(0), pk(0);
     const bool raw_out = encode_chunk<false>(
-        sm, A.sy, v, before, Y, R, R, m, pz, pk,
+        sm, A.sy, v, before, Y, R, R, m, sm.pend[0], pz, pk,
         [&]() {
-          resolve_pending(sm, src);
+          resolve_pending(sm, src, sm.pend[0]);
           park(s ^ 1);
         },
-        [&]() { write_pending<false>(sm, src, R, R); },
+        [&]() { write_pending<false>(sm, src, sm.pend[0], R, R); },
         [&](uint32_t bytes) {
           if (feeder) {
             const int cs = min(sm.st[s ^ 1].csize, CS);

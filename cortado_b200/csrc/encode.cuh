@@ -91,7 +91,7 @@ struct Packer {
 // padded (staged()), to `st`, which may be Y itself and is not written before
 // the planes have been read, or unpadded to `st_small` (not Y) when it has at
 // most SMALL bytes, and stays there until flush_staged writes it out.  The
-// chunk's size is published for the lookback and the chunk recorded in sm.pend.
+// chunk's size is published for the lookback and the chunk recorded in `pend`.
 // Returns whether the chunk is stored raw; then nothing is staged and the
 // planes are still in Y.  The caller holds a barrier after this, then every
 // thread finishes its runs pz and pk.
@@ -102,7 +102,7 @@ struct Packer {
 // the re-encoders' code short.
 template <bool KEEP, typename Written, typename Ready, typename Read>
 __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (&v)[32], uint32_t prev0, uint32_t* Y,
-                                             uint32_t* st, uint32_t* st_small, const StageMeta& m, Packer& pz, Packer& pk,
+                                             uint32_t* st, uint32_t* st_small, const StageMeta& m, Pend& pend, Packer& pz, Packer& pk,
                                              Written planes_written, Ready planes_ready, Read planes_read) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nw = m.nw;
@@ -156,7 +156,7 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
     planes_read(2u);
     if (tid == 0) {
       lookback_publish(sy, sm.epoch, m.c, 2u);
-      sm.pend = Pend{m.c, m.item, nw, 2, 0, 1, 1};
+      pend = Pend{m.c, m.item, nw, 2, 0, 1, 1};
       st_small[0] = (uint32_t)osize;
     }
     return false;
@@ -242,7 +242,7 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
     if (raw) csize = osize;
     if (tid == 0) {
       lookback_publish(sy, sm.epoch, m.c, csize);
-      sm.pend = Pend{m.c, m.item, nw, (int)csize, (int)raw, (int)small, 1};
+      pend = Pend{m.c, m.item, nw, (int)csize, (int)raw, (int)small, 1};
     }
     if (warp == 0 && !raw) {
       if (NZ == 0) {
@@ -321,14 +321,13 @@ __device__ __noinline__ void flush_words(uint8_t* dst, const uint32_t* words, in
   store_payload(dst, 4 * nw, [=](int w) -> uint32_t { return w < nw ? words[w] : 0u; });
 }
 
-// Writes out the pending chunk (its output offset in sm.payload_off; both
+// Writes out a pending chunk (p; its output offset in sm.payload_off; both
 // visible after a barrier) from its staging buffer -- or, for a raw chunk, from
 // raw_words, when not null (else its words are staged too, not padded) -- and
 // its size-table entry; the stream's last chunk also sets the stream size.
-__device__ __forceinline__ void flush_staged(const Ctl& sm, const uint32_t* st, const uint32_t* st_small,
+__device__ __forceinline__ void flush_staged(const Ctl& sm, const Pend& p, const uint32_t* st, const uint32_t* st_small,
                                              const uint32_t* raw_words, uint8_t* data_out, uint16_t* table_out,
                                              long long* out_size, long long chunks) {
-  const Pend& p = sm.pend;
   const unsigned long long X = sm.payload_off;
   if (p.raw && raw_words) {
     flush_words(data_out + X, raw_words, p.nw);

@@ -110,7 +110,7 @@ struct __align__(16) Ctl {
   uint64_t bar;             // a chunk's loads
   uint64_t bar_src;         // resi_recv: the client chunk
   StageMeta st[2];
-  Pend pend;                // encoders: the chunk whose payload waits to be flushed
+  Pend pend[2];             // encoders: the chunks whose payloads wait to be flushed
   unsigned long long payload_off;
   unsigned int epoch, is_last;
   unsigned int first;       // the CTA's first place in the queue (all ones: the helper)
