@@ -25,10 +25,12 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t s) {
   asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(s));
   return r;
 }
-// Byte-permute selectors of two bitmap nibbles m and m' = m >> 4 (the low 8
-// bits of x), see expand_sel: bit i spread to nibble i, then rank or 4 + rank
-// with one multiply-add (the multiplies run beside the logic pipe).  prmt
-// reads a selector's low 16 bits only.
+// Byte-permute selectors of two bitmap nibbles m (the low 4 bits of x) and m'
+// (the next 4): each scatters the first popc(m) bytes of a word to the positions
+// of m's set bits and zero-fills the others.  Bit i is spread to nibble i, then
+// becomes its rank, or 4 + the rank for an unset bit (a byte of the zero
+// operand), with one multiply-add; the multiplies run beside the logic pipe.
+// prmt reads a selector's low 16 bits only.
 __device__ __forceinline__ void spread_sel2(uint32_t x, uint32_t& s0, uint32_t& s1) {
   uint32_t s = (x * 0x1001u) & 0x000f000fu;
   s = (s * 0x41u) & 0x03030303u;

@@ -169,18 +169,6 @@ __device__ __forceinline__ void latch(unsigned int* status, unsigned int code) {
 }
 
 // ---------------------------------------------------------------- quantizers
-// Server quantizer (truncation), include/components/d_SQ_IABS_4.h:62-76.
-// Values below the bound's exponent give shift >= 25, which the clamping
-// shift turns into 0, so no separate test is needed.
-__device__ __forceinline__ uint32_t sq_enc(uint32_t v, const Quant& q) {
-  const uint32_t a = v & 0x7fffffffu;
-  const int ve = (int)(a >> 23);
-  const uint32_t mant = (v & 0x7fffffu) | 0x800000u;
-  const uint32_t lossy = shr_clamp(mant, (uint32_t)(q.thr_e - ve));
-  const uint32_t enc = (ve >= q.thr_e) ? a - (uint32_t)q.offs : lossy;
-  const uint32_t s = (uint32_t)((int32_t)v >> 31);
-  return (enc ^ s) - s;
-}
 // Client quantizer (round half away from zero), d_CQ_IABS_4.h:62-77.
 __device__ __forceinline__ uint32_t cq_enc(uint32_t v, const Quant& q) {
   const uint32_t a = v & 0x7fffffffu;
@@ -297,20 +285,11 @@ __device__ __forceinline__ void transpose_blocks(uint32_t (&a)[N]) {
   swap_stage<2>(a, 0x33333333u);
   swap_stage<1>(a, 0x55555555u);
 }
-__device__ __forceinline__ void transpose32(uint32_t (&a)[32]) {
-#pragma unroll
-  for (int k = 0; k < 16; k++) {
-    const uint32_t x = a[k], y = a[k + 16];
-    a[k] = __byte_perm(x, y, 0x3276);
-    a[k + 16] = __byte_perm(x, y, 0x1054);
-  }
-  transpose_blocks(a);
-}
 // Full groups are transposed one half of the planes at a time: words k and
 // k + 16 share a register (their high halves for planes 0..15, their low halves
 // for planes 16..31), and the stages run on 16 registers.  The pass for planes
 // that are zero in the whole warp is left out, and both passes are the same
-// code, half as long as transpose32.
+// code.
 
 // ---------------------------------------------------------------- byte masks
 // 4-bit mask of the non-zero bytes of x (bit b <-> byte b).
@@ -342,13 +321,6 @@ __device__ __forceinline__ uint32_t nz_nibbles8(uint32_t x) {
 __device__ __forceinline__ uint32_t nibble_at(const uint32_t (&M)[4], uint32_t k) {
   const uint32_t w = (k < 16) ? ((k < 8) ? M[0] : M[1]) : ((k < 24) ? M[2] : M[3]);
   return (w >> (4 * (k & 7))) & 15u;
-}
-// Byte-permute selector that scatters the first popc(m) bytes of a word to
-// the positions of the set bits of m and zero-fills the others.
-__device__ __forceinline__ uint32_t expand_sel(uint32_t m) {
-  const uint32_t s = (m | (m << 3) | (m << 6) | (m << 9)) & 0x1111u;
-  const uint32_t r = s * 0x1110u;
-  return (r | ((s ^ 0x1111u) << 2)) & 0xffffu;
 }
 
 // ---------------------------------------------------------------- swizzle
@@ -500,12 +472,6 @@ __device__ __forceinline__ unsigned long long lookback_published(const Sync& sy,
 __device__ __forceinline__ void lookback_publish(const Sync& sy, unsigned int epoch, long long c,
                                                  unsigned int csize) {
   st_relaxed(&sy.flags[c], ((unsigned long long)epoch << 48) | (c == 0 ? LB_INC : LB_AGG) | csize);
-}
-
-__device__ __forceinline__ unsigned long long lookback(const Sync& sy, unsigned int epoch, long long c,
-                                                       unsigned int csize) {
-  if ((threadIdx.x & 31) == 0) lookback_publish(sy, epoch, c, csize);
-  return lookback_published(sy, epoch, c, csize);
 }
 
 // Exclusive output offset of chunk c whose size was published a while ago:

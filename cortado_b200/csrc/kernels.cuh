@@ -173,46 +173,6 @@ __device__ __forceinline__ void plane_offsets(int tid, uint32_t& e, uint32_t& o)
   o = 32 * warp + ((((lane >> 2) & 7u) ^ (warp + 4)) << 2) + (lane & 3);
 }
 
-// ---------------------------------------------------------------- rotated walks
-// A thread's zero-eliminated bytes lie in a contiguous region that starts where
-// the previous thread's ended.  For dense data those regions are about 128 bytes
-// apart, so threads that walk their 32 words in the same order read the same
-// shared-memory bank.  The expansion of a dense warp therefore starts at another
-// word in every lane: nibble j of the rotated mask (rot_nibbles) belongs to word
-// (start + j) % 32, and nibble_prefix gives the byte count before the start.
-
-// Bytes before word k of a segment: the set bits of the 4-bit-per-word mask
-// M (128 bits) below nibble k.
-__device__ __forceinline__ uint32_t nibble_prefix(const uint32_t (&M)[4], int k) {
-  const int nb = 4 * k;
-  uint32_t c = 0;
-#pragma unroll
-  for (int w = 0; w < 4; w++) {
-    const int lim = nb - 32 * w;
-    const uint32_t mask = lim >= 32 ? 0xffffffffu : (lim <= 0 ? 0u : (1u << lim) - 1u);
-    c += __popc(M[w] & mask);
-  }
-  return c;
-}
-
-// The 128-bit mask M rotated right by 4*r bits.
-__device__ __forceinline__ void rot_nibbles(const uint32_t (&M)[4], int r, uint32_t (&R)[4]) {
-  uint32_t a0 = M[0], a1 = M[1], a2 = M[2], a3 = M[3];
-  if (r & 8) {
-    const uint32_t t = a0;
-    a0 = a1; a1 = a2; a2 = a3; a3 = t;
-  }
-  if (r & 16) {
-    uint32_t t = a0; a0 = a2; a2 = t;
-    t = a1; a1 = a3; a3 = t;
-  }
-  const uint32_t bs = 4 * (r & 7);
-  R[0] = __funnelshift_r(a0, a1, bs);
-  R[1] = __funnelshift_r(a1, a2, bs);
-  R[2] = __funnelshift_r(a2, a3, bs);
-  R[3] = __funnelshift_r(a3, a0, bs);
-}
-
 // The partial last chunk of a stream (nw < 4096 words, G whole groups and a
 // remainder that BIT_4 copies untransposed) runs through the full chunks' code:
 // these two move its BIT_4 output (plane s at words s*G .. s*G+G-1, then the
