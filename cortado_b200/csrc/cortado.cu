@@ -683,12 +683,15 @@ __device__ __noinline__ void client_raw_bins(const OpArgs& A, long long c, int n
 // Rebuilds a raw chunk's requantized words from the plane buffer into the
 // staging buffer, in order (out of line: only chunks that do not compress take
 // it, and the re-encoders' loop is large enough to stall on instruction fetch).
+// Only the chunk's own nw words: behind them the next payload may already be on
+// its way, since room_out() reserved no more than the chunk's bytes.
 __device__ __noinline__ void raw_rebuild(Ctl& sm, uint32_t* X, int nw, uint32_t* Yw) {
   uint32_t w[32], before;
   if (nw != CW) widen_planes(X, nw);
   planes_to_words<true>(sm, X, w, before);
 #pragma unroll
-  for (int k = 0; k < 32; k++) Yw[32 * threadIdx.x + k] = w[k];
+  for (int k = 0; k < 32; k++)
+    if (32 * (int)threadIdx.x + k < nw) Yw[32 * threadIdx.x + k] = w[k];
 }
 
 // Blocking flush of the re-encoders' pending chunk, outside the hot path: when
