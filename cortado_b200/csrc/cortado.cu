@@ -927,7 +927,10 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
         }
       }
     }
-    if (m.bad >= 2) continue;  // unusable stream header (batched): nothing to write
+    if (m.bad >= 2) {  // unusable stream header (batched): nothing to write
+      __syncthreads();  // every warp has read m.bad: the feeder may take this slot again at once
+      continue;
+    }
     uint32_t v[32];
     if (kind == CHUNK_ZERO) {
 #pragma unroll
