@@ -242,7 +242,7 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
     if (raw) csize = osize;
     if (tid == 0) {
       lookback_publish(sy, sm.epoch, m.c, csize);
-      pend = Pend{m.c, m.item, nw, (int)csize, (int)raw, (int)small, 1};
+      pend = Pend{m.c, m.item, nw, (int)csize, (int)raw, (int)(small && !raw), 1};
     }
     if (warp == 0 && !raw) {
       if (NZ == 0) {
@@ -323,7 +323,7 @@ __device__ __noinline__ void flush_words(uint8_t* dst, const uint32_t* words, in
 
 // Writes out a pending chunk (p; its output offset in sm.payload_off; both
 // visible after a barrier) from its staging buffer -- or, for a raw chunk, from
-// raw_words, when not null (else its words are staged too, not padded) -- and
+// raw_words, when not null (else its words are staged too) -- and
 // its size-table entry; the stream's last chunk also sets the stream size.
 __device__ __forceinline__ void flush_staged(const Ctl& sm, const Pend& p, const uint32_t* st, const uint32_t* st_small,
                                              const uint32_t* raw_words, uint8_t* data_out, uint16_t* table_out,
@@ -333,7 +333,7 @@ __device__ __forceinline__ void flush_staged(const Ctl& sm, const Pend& p, const
     flush_words(data_out + X, raw_words, p.nw);
   } else {
     if (p.small) st = st_small;
-    const uint32_t pad = (p.small | p.raw) ? 31 : 5;  // no padding, or staged()
+    const uint32_t pad = p.small ? 31 : 5;  // no padding, or staged()
     store_payload(data_out + X, p.csize, [&](int w) -> uint32_t { return st[(uint32_t)w + ((uint32_t)w >> pad)]; });
   }
   if (threadIdx.x == 0) {
