@@ -99,8 +99,9 @@ struct Packer {
 // which the planes are read, planes_ready() after it, and planes_read(n) after
 // the next one, with a bound n of the payload's bytes.
 // KEEP: the plane words stay in registers (st is Y); else they are read again for the packing, eight at a time in a loop, which keeps
-// the re-encoders' code short.
-template <bool KEEP, typename Written, typename Ready, typename Read>
+// the re-encoders' code short.  ZEROS: the words may all be zero (else the caller
+// has seen to such chunks).
+template <bool KEEP, bool ZEROS, typename Written, typename Ready, typename Read>
 __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (&v)[32], uint32_t prev0, uint32_t* Y,
                                              uint32_t* st, uint32_t* st_small, const StageMeta& m, Pend& pend, Packer& pz, Packer& pk,
                                              Written planes_written, Ready planes_ready, Read planes_read) {
@@ -147,7 +148,9 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
     compact_planes(Y, nw);
   }
   planes_written();
-  const bool any_nz = __syncthreads_or(any != 0);
+  bool any_nz = true;
+  if (ZEROS) any_nz = __syncthreads_or(any != 0);
+  else __syncthreads();
   planes_ready();
   if (!any_nz) {
     // No difference at all: zero elimination leaves no byte, so RZE_1 emits
