@@ -996,7 +996,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     } else if (kind == CHUNK_PLANES) {
       uint32_t before;
       planes_to_words<false>(sm, Q, v, before);
-    } else {
+    } else if (OP == OP_RAPPLY) {
       row_load(Q, tid, v);
     }
     const Quant q = make_quant(m.eb_e);
@@ -1054,8 +1054,10 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     }
     // Chunks stored uncompressed are copied out as stored: original floats for
     // storage decode (d_server_encode.h:234-249), request bins for init_recv
-    // (d_client_encode.h:230-254, the reference's behaviour).
-    if (OP == OP_RAPPLY || kind != CHUNK_RAW) {
+    // (d_client_encode.h:230-254, the reference's behaviour); they are in their
+    // places in Q already (128 MiB of random bits: init_recv 74 -> 71 us, storage
+    // decode 58 -> 56).  Zero bins are zero as floats (zeros: 34 -> 32 us).
+    if (OP == OP_RAPPLY || kind == CHUNK_PLANES) {
       // The float form holds for bins up to 2^23 in magnitude (that one is
       // the lossless threshold itself in both forms).
       float f[32], fmax = 0.0f;
@@ -1073,7 +1075,8 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
         for (int k = 0; k < 32; k++) v[k] = iq_mixed(v[k], fq, q);
       }
     }
-    row_store(Q, tid, v);  // every plane read finished before the decoder's last barrier
+    if (OP == OP_RAPPLY || kind != CHUNK_RAW)
+      row_store(Q, tid, v);  // every plane read finished before the decoder's last barrier
     const bool tma_out = full && A.has_map_out;
     if (tma_out) fence_proxy_async();
     __syncthreads();
