@@ -131,8 +131,8 @@ struct NoHook {
 
 // Writes `csize` payload bytes to global memory at dst (any alignment) with
 // 16-byte stores for the aligned interior.  word(q) returns payload word q
-// (bytes 4q..4q+3, little-endian).
-template <typename WordFn>
+// (bytes 4q..4q+3, little-endian).  UNROLL: blocks in flight per thread.
+template <int UNROLL = 1, typename WordFn>
 __device__ __forceinline__ void store_payload(uint8_t* dst, int csize, WordFn word) {
   const int tid = threadIdx.x;
   const uintptr_t A = reinterpret_cast<uintptr_t>(dst);
@@ -143,6 +143,7 @@ __device__ __forceinline__ void store_payload(uint8_t* dst, int csize, WordFn wo
     const int head = (int)(a0 - A);
     const int nblk = (int)((a1 - a0) >> 4);
     const int r = head & 3;
+#pragma unroll(UNROLL)
     for (int b = tid; b < nblk; b += NT) {
       const int o = head + 16 * b;
       const int q = o >> 2;
