@@ -1221,11 +1221,8 @@ __device__ __forceinline__ bool maxabs_bad(float o, float r, float eb) {
 
 // Bound by DRAM (both arrays once): four pairs of 16-byte loads in flight per
 // thread where both arrays allow it (2 x 512 MiB: 280 -> 163 us, 6.6 TB/s; one
-// pair of 4-byte loads kept too little in flight).  Plain loads: the arrays were
-// often written just before and may lie in L2, where streaming loads lose them
-// (2 x 32 MiB checked again: 16.6 us with them, 12.5 without; large arrays the
-// same).  A thread stops at its first violation, which is the lowest of its
-// indices.
+// pair of 4-byte loads kept too little in flight).  A thread stops at its first
+// violation, which is the lowest of its indices.
 __global__ void __launch_bounds__(256) k_verify(const float* __restrict__ orig, const float* __restrict__ recon, long long nw, float eb,
                          unsigned long long* first_bad) {
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -1239,8 +1236,8 @@ __global__ void __launch_bounds__(256) k_verify(const float* __restrict__ orig, 
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const long long k = min(i + j * stride, nv - 1);  // (the last one again: it changes nothing)
-      o[j] = __ldg(o4 + k);
-      r[j] = __ldg(r4 + k);
+      o[j] = __ldcs(o4 + k);
+      r[j] = __ldcs(r4 + k);
     }
     bool bad = false;
 #pragma unroll
