@@ -691,6 +691,25 @@ __device__ __noinline__ void client_raw_bins(const OpArgs& A, long long c, int n
     if (32 * tid + k < nw) row[k] = Yw[staged(32 * tid + k)];
 }
 
+// The fused forms for a chunk of zeros: request bins of zero are zero as floats;
+// residuals of zero move the client's floats to the destination bound's bins.
+template <int OP>
+__device__ __noinline__ void client_zero(const OpArgs& A, long long c, int nw, Quant q) {
+  const FastQ fq = make_fastq(q.eb_e);
+  uint32_t* client = reinterpret_cast<uint32_t*>(A.client) + c * (long long)CW;
+  auto moved = [&](uint32_t x) -> uint32_t { return (OP == OP_S2C) ? 0u : iq_mixed(cq_mixed(x, fq, q), fq, q); };
+  if (nw == CW) {
+    uint4* g4 = reinterpret_cast<uint4*>(client) + threadIdx.x;
+#pragma unroll 2
+    for (int i = 0; i < 8; i++) {
+      const uint4 w = (OP == OP_S2C) ? make_uint4(0, 0, 0, 0) : g4[NT * i];
+      g4[NT * i] = make_uint4(moved(w.x), moved(w.y), moved(w.z), moved(w.w));
+    }
+  } else {
+    for (int w = threadIdx.x; w < nw; w += NT) client[w] = moved((OP == OP_S2C) ? 0u : client[w]);
+  }
+}
+
 // Rebuilds a raw chunk's requantized words from the plane buffer into the
 // staging buffer, padded as payloads are (staged(): a thread's words start 33
 // words from the next one's, so no two lanes meet in a bank; unpadded, init_send
@@ -800,16 +819,13 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
       if (feeder) issue(s ^ 1);
       continue;
     }
-    if (OP == OP_S2C && kind == CHUNK_ZERO) {  // request bins and the client's floats are zero as well
+    if ((OP == OP_S2C || APPLY) && kind == CHUNK_ZERO) {  // request bins and residuals are zero as well
       resolve(s ^ 1, g);
       park(s ^ 1);
       Quant q1, q2;
       src.quant(m.item, q1, q2);
-      if (Src::batched && m.c == 0 && tid == 0) write_header(A.out, m.n, q1.eb_e);
-      if (APPLY && A.client) {
-        uint32_t* client = reinterpret_cast<uint32_t*>(A.client) + m.c * (long long)CW;
-        for (int w = tid; w < m.nw; w += NT) client[w] = 0;
-      }
+      if (Src::batched && m.c == 0 && tid == 0) write_header(A.out, m.n, (OP == OP_S2C) ? q1.eb_e : q2.eb_e);
+      if (APPLY && A.client) client_zero<OP>(A, m.c, m.nw, q2);
       zero_chunk(sm, src, m, R);
       if (feeder) issue(s ^ 1);
       continue;
@@ -825,7 +841,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
       before = tid ? Y[swz(32 * tid - 1)] : 0u;
       __syncthreads();  // rows are scratch from here on
     }
-    uint32_t some = 0;  // resi_send: bits set in this thread's residuals
+    uint32_t some = 0;  // plain resi_send: bits set in this thread's residuals
     {
       // stored bins -> floats (iSQ, skipped for chunks stored as floats) ->
       // request bins (CQ, d_s2c.h:132-137) or residuals (d_RESI_4.h:57-76)
@@ -871,7 +887,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
           before = requant_words<OP>(Y, slow, before, slow_before, raw, qs, q1, q2);
           row_load(Y, tid, v);
         }
-        if (OP == OP_RESI) {
+        if (OP == OP_RESI && !APPLY) {
 #pragma unroll
           for (int k = 0; k < 32; k++) some |= v[k];
         }
@@ -881,7 +897,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
       if (APPLY && A.client) client_apply<OP>(A, m.c, m.nw, v, OP == OP_S2C ? q1 : q2, Y);
     }
     // (the rows of Y are free after the barrier)
-    if (OP != OP_RESI) {
+    if (OP == OP_S2C || APPLY) {
       __syncthreads();
     } else if (!__syncthreads_or(some != 0)) {
       park(s ^ 1);
@@ -890,7 +906,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
       continue;
     }
     Packer pz(0), pk(0);
-    const bool raw_out = encode_chunk<false, OP == OP_S2C>(
+    const bool raw_out = encode_chunk<false, OP == OP_S2C || APPLY>(
         sm, A.sy, v, before, Y, R, R, m, sm.pend[0], pz, pk,
         [&]() {
           resolve_pending(sm, src, sm.pend[0]);
