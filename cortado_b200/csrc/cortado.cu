@@ -1240,9 +1240,11 @@ __device__ __forceinline__ bool maxabs_bad(float o, float r, float eb) {
 }
 
 // Bound by DRAM (both arrays once): four pairs of 16-byte loads in flight per
-// thread where both arrays allow it (2 x 512 MiB: 280 -> 163 us, 6.6 TB/s; one
-// pair of 4-byte loads kept too little in flight).  A thread stops at its first
-// violation, which is the lowest of its indices.
+// thread where both arrays allow it (2 x 512 MiB: 277 -> 162 us, 6.6 TB/s; one
+// pair of 4-byte loads kept too little in flight), eight pairs of 4-byte loads
+// where not (500 us with one pair in this kernel, 273 in one of its own with
+// more warps per SM, 192 now).  A thread stops at its first violation, which is
+// the lowest of its indices.
 __global__ void __launch_bounds__(256) k_verify(const float* __restrict__ orig, const float* __restrict__ recon, long long nw, float eb,
                          unsigned long long* first_bad) {
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -1276,10 +1278,26 @@ __global__ void __launch_bounds__(256) k_verify(const float* __restrict__ orig, 
       }
     }
   }
-  for (long long i = 4 * nv + t; i < nw; i += stride) {
-    if (maxabs_bad(orig[i], recon[i], eb)) {
-      atomicMin(first_bad, (unsigned long long)i);
-      return;
+  for (long long i = 4 * nv + t; i < nw; i += 8 * stride) {
+    float o[8], r[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const long long k = min(i + j * stride, nw - 1);
+      o[j] = orig[k];
+      r[j] = recon[k];
+    }
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < 8; j++) bad |= maxabs_bad(o[j], r[j], eb);
+    if (bad) {
+#pragma unroll 1
+      for (int j = 0; j < 8; j++) {
+        const long long k = min(i + j * stride, nw - 1);
+        if (maxabs_bad(orig[k], recon[k], eb)) {
+          atomicMin(first_bad, (unsigned long long)k);
+          return;
+        }
+      }
     }
   }
 }
