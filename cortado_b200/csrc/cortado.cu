@@ -814,7 +814,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
     const StageMeta& m = sm.st[s];
     if (m.g >= src.total) break;
     const OpArgs& A = src.args(m.item);
-    const ChunkKind kind = rze_decode(sm, A.sy, m, R, Y, NoHook{});
+    const ChunkKind kind = rze_decode<true>(sm, A.sy, m, R, Y, NoHook{});
     const unsigned int g = take();
     if (m.bad >= 2) {  // unusable stream header (batched): nothing to write
       resolve(s ^ 1, g);
@@ -988,7 +988,36 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     auto q_free = [&]() {
       if (tid == TMA_TID) bulk_wait_read();  // the previous chunk's TMA store has read Q
     };
-    const ChunkKind kind = rze_decode(sm, A.sy, m, P, Q, q_free);
+    if (OP != OP_RAPPLY && m.csize == 4 * nw) {
+      // Stored uncompressed: copied out as stored, original floats for storage
+      // decode (d_server_encode.h:234-249), request bins for init_recv
+      // (d_client_encode.h:230-254, the reference's behaviour).  Q is not
+      // needed, so the next payload is loaded there at once and the buffers
+      // change places: nothing but that load would hide its latency.  The load
+      // may complete the barrier's next phase, so the feeder first waits until
+      // every warp has seen this one.
+      if (feeder) {
+        q_free();
+        park_stream(sm, s ^ 1, src, ah);
+        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+        issue_stream(sm, s ^ 1, src, reinterpret_cast<uint8_t*>(Q), 0);
+      } else {
+        asm volatile("bar.arrive 1, %0;" ::"n"(NT) : "memory");
+      }
+      uint32_t* g = reinterpret_cast<uint32_t*>(A.out) + c * (long long)CW;
+      const int d = m.d;
+#pragma unroll 4
+      for (int w = tid; w < nw; w += NT) {
+        const int o = d + 4 * w;
+        g[w] = __funnelshift_r(P[o >> 2], P[(o >> 2) + 1], 8 * (o & 3));
+      }
+      uint32_t* const t = P;
+      P = Q;
+      Q = t;
+      __syncthreads();  // the payload and the slot have been read
+      continue;
+    }
+    const ChunkKind kind = rze_decode<OP == OP_RAPPLY>(sm, A.sy, m, P, Q, q_free);
     if (feeder) {
       park_stream(sm, s ^ 1, src, ah);
       issue_stream(sm, s ^ 1, src, reinterpret_cast<uint8_t*>(P), 0);
@@ -1072,11 +1101,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
         }
       }
     }
-    // Chunks stored uncompressed are copied out as stored: original floats for
-    // storage decode (d_server_encode.h:234-249), request bins for init_recv
-    // (d_client_encode.h:230-254, the reference's behaviour); they are in their
-    // places in Q already (128 MiB of random bits: init_recv 74 -> 71 us, storage
-    // decode 58 -> 56).  Zero bins are zero as floats (zeros: 34 -> 32 us).
+    // (Zero bins are zero as floats: 128 MiB of zeros 34 -> 32 us.)
     if (OP == OP_RAPPLY || kind == CHUNK_PLANES) {
       // The float form holds for bins up to 2^23 in magnitude (that one is
       // the lossless threshold itself in both forms).
@@ -1095,8 +1120,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
         for (int k = 0; k < 32; k++) v[k] = iq_mixed(v[k], fq, q);
       }
     }
-    if (OP == OP_RAPPLY || kind != CHUNK_RAW)
-      row_store(Q, tid, v);  // every plane read finished before the decoder's last barrier
+    row_store(Q, tid, v);  // every plane read finished before the decoder's last barrier
     const bool tma_out = full && A.has_map_out;
     if (tma_out) fence_proxy_async();
     __syncthreads();

@@ -97,7 +97,8 @@ enum ChunkKind : int { CHUNK_ZERO = 0, CHUNK_PLANES = 1, CHUNK_RAW = 2 };
 // 90 instructions), so no warp waits for another before the level-1 bitmap
 // (warp 0 decoding them for the others took a barrier and left three warps
 // idle meanwhile).
-template <typename Free>
+// RAW: the chunk may be stored uncompressed (else the caller has seen to such chunks).
+template <bool RAW, typename Free>
 __device__ __forceinline__ ChunkKind rze_decode(Ctl& sm, const Sync& sy, const StageMeta& m, const uint32_t* P,
                                                 uint32_t* Q, Free q_free) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -111,7 +112,7 @@ __device__ __forceinline__ ChunkKind rze_decode(Ctl& sm, const Sync& sy, const S
     __syncthreads();
     return CHUNK_ZERO;
   }
-  if (csize == osize) {  // stored uncompressed: realigned words
+  if (RAW && csize == osize) {  // stored uncompressed: realigned words
     q_free();
     __syncthreads();
 #pragma unroll 4
