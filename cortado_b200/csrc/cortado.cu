@@ -68,6 +68,7 @@ __device__ __forceinline__ bool begin_launch(Ctl& sm, const Sync& sy) {
     sm.epoch = e;
     sm.first = p;
     sm.pend[0].valid = sm.pend[1].valid = 0;
+    sm.zeros = 0;
   }
   if (threadIdx.x == TMA_TID) {
     mbar_init(&sm.bar, 2);
@@ -337,8 +338,8 @@ __device__ __forceinline__ void write_pending(Ctl& sm, const Src& src, const Pen
   if (!pd.valid) return;
   const OpArgs& Q = src.args(pd.item);
   const long long chunks = (Q.n + CS - 1) / CS;
-  flush_staged(sm, pd, st, st_small, FLOATS ? reinterpret_cast<const uint32_t*>(Q.in) + pd.c * (long long)CW : nullptr,
-               Q.out + HDR + 2 * chunks, reinterpret_cast<uint16_t*>(Q.out + HDR), Q.out_size, chunks);
+  flush_staged<FLOATS>(sm, pd, st, st_small, FLOATS ? reinterpret_cast<const uint32_t*>(Q.in) + pd.c * (long long)CW : nullptr,
+                       Q.out + HDR + 2 * chunks, reinterpret_cast<uint16_t*>(Q.out + HDR), Q.out_size, chunks);
 }
 
 // store (d_server_encode_kernel): floats -> SQ -> encode.  One buffer (A)
@@ -589,7 +590,7 @@ __device__ __forceinline__ void issue_stream(Ctl& sm, int t, const Src& src, uin
 // init_recv / resi_recv of that stream bit for bit:
 //   init: iCQ(bin) (d_client_encode.h:230-254); a chunk that the encoder
 //         stores uncompressed is rewritten with its bins afterwards
-//         (client_raw_bins), as init_recv copies raw chunks out as stored;
+//         (raw_rebuild), as init_recv copies raw chunks out as stored;
 //   resi: iCQ(CQ(client, dst) + residual, dst) (d_RESI_4.h:79-94); the
 //         residual ints are the same whether the chunk compresses or not.
 // A full chunk goes through the stage buffer X, whose rows 32w .. 32w+31
@@ -685,16 +686,6 @@ __device__ __forceinline__ void client_apply(const OpArgs& A, long long c, int n
   }
 }
 
-// init_send with apply, for a chunk stored uncompressed: its bins (rebuilt in
-// Yw by raw_rebuild) replace the dequantized words this thread wrote, as
-// init_recv emits a raw chunk's bins unchanged.
-__device__ __noinline__ void client_raw_bins(const OpArgs& A, long long c, int nw, const uint32_t* Yw) {
-  const int tid = threadIdx.x;
-  uint32_t* row = reinterpret_cast<uint32_t*>(A.client) + c * (long long)CW + 32 * tid;
-  for (int k = 0; k < 32; k++)
-    if (32 * tid + k < nw) row[k] = Yw[staged(32 * tid + k)];
-}
-
 // The fused forms for a chunk of zeros: request bins of zero are zero as floats;
 // residuals of zero move the client's floats to the destination bound's bins.
 template <int OP>
@@ -714,48 +705,156 @@ __device__ __noinline__ void client_zero(const OpArgs& A, long long c, int nw, Q
   }
 }
 
-// Rebuilds a raw chunk's requantized words from the plane buffer into the
-// staging buffer, padded as payloads are (staged(): a thread's words start 33
-// words from the next one's, so no two lanes meet in a bank; unpadded, init_send
-// took 312 us instead of 252 on 128 MiB of random bits, init_send_apply 498
-// instead of 356).  Out of line: only chunks that do not compress take it, and
-// the re-encoders' loop is large enough to stall on instruction fetch.
-// Only the chunk's own nw words: behind them the next payload may already be on
-// its way, since room_out() reserved no more than the chunk's bytes.
-__device__ __noinline__ void raw_rebuild(Ctl& sm, uint32_t* X, int nw, uint32_t* Yw) {
+// Bytes of the re-encoders' R (reencode_loop).
+constexpr int ROOM = (2 * BUF_WORDS - CW) * 4;
+// Bytes that a payload of n bytes takes at R's high end (any alignment, and
+// what the decoder reads past its end), and at its low end (padded).
+__host__ __device__ constexpr int room_in(int n) { return ((n + 30) & ~15) + 32; }
+__host__ __device__ constexpr int room_out(int n) { return n + (n >> 5) + 32; }
+static_assert(room_out(SMALL) + room_in(CS) <= ROOM, "a payload that is not padded is never spilled");
+static_assert(room_out(CS) <= 4 * BUF_WORDS, "a payload fits the CTA's place in global memory");
+
+// Rebuilds a raw chunk's requantized words from the planes (X) and spills them.
+// Each warp moves its 4 KiB through its own rows of X, 512 contiguous bytes at a
+// time.  client (init_send with apply, or null): the chunk's bins replace the
+// dequantized words written there, as init_recv emits a raw chunk's bins
+// unchanged.  Out of line: only chunks that do not compress take it, and the
+// re-encoders' loop is large enough to stall on instruction fetch.
+__device__ __noinline__ void raw_rebuild(Ctl& sm, uint32_t* X, int nw, uint32_t* spill, uint32_t* client) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t w[32], before;
   if (nw != CW) widen_planes(X, nw);
   planes_to_words<true>(sm, X, w, before);
-#pragma unroll
-  for (int k = 0; k < 32; k++)
-    if (32 * (int)threadIdx.x + k < nw) Yw[staged(32 * threadIdx.x + k)] = w[k];
+  row_store(X, tid, w);
+  if (tid == 0) {
+    sm.pend[1] = sm.pend[0];
+    sm.pend[0].valid = 0;
+  }
+  __syncwarp();
+  const uint4* X4 = reinterpret_cast<const uint4*>(X);
+#pragma unroll 2
+  for (int i = 0; i < 8; i++) {
+    const int r = 32 * warp + 4 * i + (lane >> 3), u = 256 * warp + 32 * i + lane;
+    const uint4 x = X4[8 * r + ((lane & 7) ^ (r & 7))];
+    __stcg(reinterpret_cast<uint4*>(spill) + u, x);
+    if (client) {
+      if (4 * u + 4 <= nw) {
+        reinterpret_cast<uint4*>(client)[u] = x;
+      } else {
+        if (4 * u < nw) client[4 * u] = x.x;
+        if (4 * u + 1 < nw) client[4 * u + 1] = x.y;
+        if (4 * u + 2 < nw) client[4 * u + 2] = x.z;
+      }
+    }
+  }
 }
 
-// Blocking flush of the re-encoders' pending chunk, outside the hot path: when
-// the next payload does not fit beside it and at the end of the loop.  Every earlier write to R may precede it without a barrier.
+// Writes out a spilled payload (pend[1]); every thread.
 template <class Src>
-__device__ __noinline__ void flush_now(Ctl& sm, const Src src, uint32_t* R) {
+__device__ __noinline__ void flush_spilled(Ctl& sm, const Src src, const uint32_t* spill) {
+  const Pend& p = sm.pend[1];
+  const OpArgs& Q = src.args(p.item);
+  const long long chunks = (Q.n + CS - 1) / CS;
+  if (threadIdx.x < 32) {
+    const unsigned long long X = lookback_resolve(Q.sy, sm.epoch, p.c, p.csize);
+    if (threadIdx.x == 0) sm.payload_off = X;
+  }
+  __syncthreads();
+  const unsigned long long X = sm.payload_off;
+  uint8_t* dst = Q.out + HDR + 2 * chunks + X;
+  if (p.raw) flush_raw(dst, spill, p.csize);
+  else flush_words<false>(dst, spill, p.csize);
+  if (threadIdx.x == 0) {
+    reinterpret_cast<uint16_t*>(Q.out + HDR)[p.c] = (uint16_t)p.csize;
+    if (p.c == chunks - 1) *Q.out_size = HDR + 2 * chunks + (long long)(X + p.csize);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) sm.pend[1].valid = 0;
+}
+
+// Blocking flush of all that is pending, outside the hot path.  Every earlier
+// write to R may precede it without a barrier.
+template <class Src>
+__device__ __noinline__ void flush_now(Ctl& sm, const Src src, uint32_t* R, const uint32_t* spill) {
   __syncthreads();
   resolve_pending(sm, src, sm.pend[0]);
   __syncthreads();
   write_pending<false>(sm, src, sm.pend[0], R, R);
   __syncthreads();
   if (threadIdx.x == 0) sm.pend[0].valid = 0;
+  if (sm.pend[1].valid) flush_spilled(sm, src, spill);
 }
 
-// A chunk whose words to encode are all zero, without the encode stage: only the
-// 2-byte trailer, the chunk's size published before the pending chunk's offset
-// is waited for.  Out of line, and init_send tells such chunks by their stored
-// bins alone: with one more live value in its loop it ran 2-5% slower.  (128 MiB
-// of zeros through the whole loop: init_send 65 -> 49 us, resi_send 70 -> 51.)
-template <class Src>
-__device__ __noinline__ void zero_chunk(Ctl& sm, const Src src, const StageMeta& m, uint32_t* R) {
-  if (threadIdx.x == 0) lookback_publish(src.args(m.item).sy, sm.epoch, m.c, 2u);
-  flush_now(sm, src, R);
+// Moves the pending payload (padded, at the low end of R) to the CTA's place in
+// global memory: the next one does not fit beside it.
+// (Waiting for the pending offset instead, to write the payload out, let CTAs
+// that had already taken their next chunk wait for one another.  128 MiB,
+// init_send: chunks of zeros and random bits mixed 288 -> 203 us, smooth and
+// random 332 -> 243, dense 273 -> 247.)
+__device__ __noinline__ void spill_now(Ctl& sm, const uint32_t* R, uint32_t* spill) {
+  __syncthreads();
+  const int n = room_out(sm.pend[0].csize) >> 4;
+  const uint4* r = reinterpret_cast<const uint4*>(R);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += NT) __stcg(reinterpret_cast<uint4*>(spill) + i, r[i]);
   if (threadIdx.x == 0) {
-    sm.pend[0] = Pend{m.c, m.item, m.nw, 2, 0, 1, 1};
-    R[0] = 4u * m.nw;
+    sm.pend[1] = sm.pend[0];
+    sm.pend[0].valid = 0;
   }
+  __syncthreads();
+}
+
+// Chunks whose words to encode are all zero go without the encode stage: their
+// sizes are published at once, and one warp (ZERO_WARP) keeps them until there
+// are 32 and then writes their 2-byte payloads, so that no other chunk waits.
+// Out of line, and init_send tells such chunks by their stored bins alone: with
+// one more live value in its loop it ran 2-5% slower.
+constexpr int ZERO_WARP = 2;
+template <class Src>
+__device__ __noinline__ void zero_flush(Ctl& sm, const Src src) {
+  const int lane = threadIdx.x & 31;
+  const bool mine = lane < (int)sm.zeros;
+  const uint32_t c = mine ? sm.zero_c[lane] : 0u;
+  const int item = mine ? sm.zero_item[lane] : 0;
+  auto write = [&](uint32_t k, int it, unsigned long long X) {
+    const OpArgs& A = src.args(it);
+    const long long chunks = (A.n + CS - 1) / CS;
+    const uint32_t osize = (uint32_t)min((long long)CS, A.n - k * (long long)CS);
+    uint8_t* dst = A.out + HDR + 2 * chunks + X;
+    dst[0] = (uint8_t)osize;
+    dst[1] = (uint8_t)(osize >> 8);
+    reinterpret_cast<uint16_t*>(A.out + HDR)[k] = 2;
+    if (k == chunks - 1) *A.out_size = HDR + 2 * chunks + (long long)X + 2;
+  };
+  bool open = false;  // the offset is not known yet
+  if (mine) {
+    const unsigned long long f = ld_relaxed(&src.args(item).sy.flags[c]);
+    if ((f >> 48) == sm.epoch && (f & LB_INC)) write(c, item, (f & LB_VAL) - 2);
+    else open = true;
+  }
+  for (unsigned int todo = __ballot_sync(0xffffffffu, open); todo; todo &= todo - 1) {
+    const int l = __ffs(todo) - 1;
+    const uint32_t k = __shfl_sync(0xffffffffu, c, l);
+    const int it = __shfl_sync(0xffffffffu, item, l);
+    const unsigned long long X = lookback_resolve(src.args(it).sy, sm.epoch, k, 2u);
+    if (lane == 0) write(k, it, X);
+  }
+  __syncwarp();
+  if (lane == 0) sm.zeros = 0;
+  __syncwarp();
+}
+// (ZERO_WARP)
+template <class Src>
+__device__ __noinline__ void zero_chunk(Ctl& sm, const Src src, const StageMeta& m) {
+  if ((threadIdx.x & 31) == 0) {
+    lookback_publish(src.args(m.item).sy, sm.epoch, m.c, 2u);
+    const unsigned int n = sm.zeros;
+    sm.zero_c[n] = (uint32_t)m.c;
+    sm.zero_item[n] = m.item;
+    sm.zeros = n + 1;
+  }
+  __syncwarp();
+  if (sm.zeros == 32) zero_flush(sm, src);
 }
 
 // init_send / resi_send (d_s2c_encode_kernel, d_residual_encode_kernel):
@@ -766,8 +865,9 @@ __device__ __noinline__ void zero_chunk(Ctl& sm, const Src src, const StageMeta&
 // chunk's new payload at the low end, until it is flushed while the new planes
 // are read, and the stored payload at the high end; the next one is loaded
 // there as soon as this chunk's size is known, or, when the two do not fit,
-// after a blocking flush.  A chunk that does not compress stores its
-// requantized words, which are rebuilt from the planes (planes_to_words).
+// after the new payload has been spilled to global memory.  A chunk that does not
+// compress stores its requantized words, which are rebuilt from the planes
+// (planes_to_words) and always spilled.
 // (Decoding in place in one buffer and staging in the other took 11 barriers a
 // chunk; this takes 7.  256 MiB: init_send 462 -> 320 us and resi_send 468 ->
 // 340 us on sinusoids with noise, 552 -> 414 and 516 -> 387 us on dense data,
@@ -777,12 +877,6 @@ __device__ __noinline__ void zero_chunk(Ctl& sm, const Src src, const StageMeta&
 // resi_send to 320, 370 and 266 us.)
 // APPLY: the fused send-and-apply forms (items with a client's floats); the
 // plain forms are compiled without that code.
-constexpr int ROOM = (2 * BUF_WORDS - CW) * 4;  // bytes of R
-// Bytes that a payload of n bytes takes at R's high end (any alignment, and
-// what the decoder reads past its end), and at its low end (padded).
-__device__ __forceinline__ int room_in(int n) { return ((n + 30) & ~15) + 32; }
-__device__ __forceinline__ int room_out(int n) { return n + (n >> 5) + 32; }
-
 template <int OP, bool APPLY, class Src>
 __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Sync& sy) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -793,6 +887,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
   }
   uint32_t* Y = stage_buf(sm, 0);
   uint32_t* R = Y + CW;
+  uint32_t* spill = sy.spill + (size_t)blockIdx.x * BUF_WORDS;
   const bool feeder = warp == 1;  // (warp 3 packs the densest planes: 1% slower)
   WalkState ws{-1};
   Ahead ah{0, 0};
@@ -819,19 +914,26 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
     if (m.bad >= 2) {  // unusable stream header (batched): nothing to write
       resolve(s ^ 1, g);
       park(s ^ 1);
-      flush_now(sm, src, R);
+      flush_now(sm, src, R, spill);
       if (feeder) issue(s ^ 1);
       continue;
     }
+    // The rest of a chunk whose words to encode are all zero.  A payload in R is
+    // written out first: CTAs that ran ahead past such chunks made the others wait
+    // (sparse fields with 2% of them: init_send 3-5% slower).  A spilled one waits.
+    auto zero = [&]() {
+      if (warp == ZERO_WARP) zero_chunk(sm, src, m);
+      park(s ^ 1);
+      if (sm.pend[0].valid) flush_now(sm, src, R, spill);
+      if (feeder) issue(s ^ 1);
+    };
     if ((OP == OP_S2C || APPLY) && kind == CHUNK_ZERO) {  // request bins and residuals are zero as well
       resolve(s ^ 1, g);
-      park(s ^ 1);
       Quant q1, q2;
       src.quant(m.item, q1, q2);
       if (Src::batched && m.c == 0 && tid == 0) write_header(A.out, m.n, (OP == OP_S2C) ? q1.eb_e : q2.eb_e);
       if (APPLY && A.client) client_zero<OP>(A, m.c, m.nw, q2);
-      zero_chunk(sm, src, m, R);
-      if (feeder) issue(s ^ 1);
+      zero();
       continue;
     }
     uint32_t v[32], before = 0;  // before: the word before this thread's first
@@ -904,9 +1006,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
     if (OP == OP_S2C || APPLY) {
       __syncthreads();
     } else if (!__syncthreads_or(some != 0)) {
-      park(s ^ 1);
-      zero_chunk(sm, src, m, R);
-      if (feeder) issue(s ^ 1);
+      zero();
       continue;
     }
     Packer pz(0), pk(0);
@@ -921,23 +1021,24 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
           if (feeder) {
             const int cs = min(sm.st[s ^ 1].csize, CS);
             const bool fits = room_out(min((int)bytes, CS)) + room_in(cs) <= ROOM;
-            if (lane == 0) sm.held = !fits;
+            if (lane == 0) sm.held = (fits ? 0u : 1u) | (sm.pend[1].valid ? 2u : 0u);
             if (fits) issue(s ^ 1);
           }
         });
-    if (raw_out) {
-      raw_rebuild(sm, Y, m.nw, R);
-      if (OP == OP_S2C && APPLY && A.client) client_raw_bins(A, m.c, m.nw, R);
-    }
     __syncthreads();  // the payload's full words are in place
     pz.finish(R);
     pk.finish(R);
-    if (sm.held) {
-      flush_now(sm, src, R);
-      if (feeder) issue(s ^ 1);
+    if (raw_out || sm.held) {
+      if (sm.held & 2u) flush_spilled(sm, src, spill);
+      if (!raw_out && (sm.held & 1u)) spill_now(sm, R, spill);
+      if (feeder && (sm.held & 1u)) issue(s ^ 1);  // (R is free: of a raw chunk nothing is staged)
+      if (raw_out)
+        raw_rebuild(sm, Y, m.nw, spill,
+                    OP == OP_S2C && APPLY && A.client ? reinterpret_cast<uint32_t*>(A.client) + m.c * (long long)CW : nullptr);
     }
   }
-  flush_now(sm, src, R);
+  if (warp == ZERO_WARP) zero_flush(sm, src);
+  flush_now(sm, src, R, spill);
 }
 
 // storage decode / init_recv / resi_recv (d_server_decode_kernel,
@@ -1415,12 +1516,21 @@ __global__ void k_wait_selftest(Sync sy) {
 }  // namespace
 
 // ================================================================== host side
+// A payload's room per CTA of a re-encoder's largest grid, in device memory.
+struct SpillRoom {
+  uint32_t* p = nullptr;
+  size_t bytes = 0;
+  int device = 0;
+  unsigned long long context = 0;
+};
+
 struct cortado_ctx {
   int device = 0;
   int sms = 0;
   int grid_store = 0, grid_reenc = 0, grid_dec = 0, grid_rapply = 0;
   unsigned long long* flags = nullptr;
   long long flags_cap = 0;
+  SpillRoom spill;
   unsigned int* words = nullptr;  // [0] queue, [1] finished, [2] status, [3..4] minmax, [5] epoch, [7] range blocks finished
   int grid_batch[6] = {0, 0, 0, 0, 0, 0};
   int ctas_override[6] = {0, 0, 0, 0, 0, 0};  // per op: resident CTAs per SM (0 = occupancy limit)
@@ -1538,6 +1648,7 @@ Sync next_sync(cortado_ctx* ctx, cudaStream_t, int op = 0) {
   s.epoch = ctx->words + 5;
   s.timeout_ns = ctx->timeout_ns;
   s.resolver = ctx->resolver[op];
+  s.spill = ctx->spill.p;
   return s;
 }
 
@@ -1607,6 +1718,77 @@ cortado_status cortado_eb_exponent(float eb, int* biased_exponent) {
   return s;
 }
 
+// The calling thread's current CUDA context (driver entry point, as for the
+// tensor-map encoder), or null when it cannot be queried.
+static CUcontext current_context() {
+  using Fn = CUresult (*)(CUcontext*);
+  static Fn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<Fn>(p);
+  });
+  CUcontext c = nullptr;
+  if (!fn || fn(&c) != CUDA_SUCCESS) return nullptr;
+  return c;
+}
+
+// The current context's id, never used again in this process, or 0.
+static unsigned long long current_context_id() {
+  using Fn = CUresult (*)(CUcontext, unsigned long long*);
+  static Fn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<Fn>(p);
+  });
+  const CUcontext c = current_context();
+  unsigned long long id = 0;
+  return c && fn && fn(c, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+// Spill rooms of destroyed contexts, up to four, for the next ones: allocating
+// one takes 0.4 to 3 ms, creating a context otherwise 0.1.  A room is used again
+// only in the CUDA context that it was allocated in (a device reset or another
+// context has another id), and the device has been waited for before it is here.
+static SpillRoom g_idle_rooms[4];
+static std::mutex g_idle_mu;
+
+static cudaError_t take_room(SpillRoom* room, int device, size_t bytes) {
+  const unsigned long long id = current_context_id();
+  if (id) {
+    std::lock_guard<std::mutex> lock(g_idle_mu);
+    for (SpillRoom& r : g_idle_rooms) {
+      if (r.p && r.bytes == bytes && r.device == device && r.context == id) {
+        *room = r;
+        r = SpillRoom{};
+        return cudaSuccess;
+      }
+    }
+  }
+  *room = SpillRoom{nullptr, bytes, device, id};
+  return cudaMalloc(&room->p, bytes);
+}
+static void give_room(const SpillRoom& room, bool reusable) {
+  if (!room.p) return;
+  if (reusable && room.context && room.context == current_context_id()) {
+    std::lock_guard<std::mutex> lock(g_idle_mu);
+    for (SpillRoom& r : g_idle_rooms) {
+      if (!r.p) {
+        r = room;
+        return;
+      }
+    }
+  }
+  cudaFree(room.p);
+}
+
 cortado_status cortado_create(cortado_ctx** out, int device) {
   if (!out) return CORTADO_ERR_INVALID_ARG;
   *out = nullptr;
@@ -1637,8 +1819,11 @@ cortado_status cortado_create(cortado_ctx** out, int device) {
   ctx->grid_batch[OP_SDEC] = occupancy_grid(k_batch<OP_SDEC>, SMEM_STD, ctx->sms);
   ctx->grid_batch[OP_CDEC] = occupancy_grid(k_batch<OP_CDEC>, SMEM_STD, ctx->sms);
   ctx->grid_batch[OP_RAPPLY] = occupancy_grid(k_batch<OP_RAPPLY>, SMEM_STD, ctx->sms);
+  int ctas = ctx->grid_reenc;
+  for (int op : {OP_S2C, OP_RESI}) ctas = ctx->grid_batch[op] > ctas ? ctx->grid_batch[op] : ctas;
   for (cudaEvent_t& ev : ctx->items_done) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-  cortado_status s = ensure_flags(ctx, 1024, 0);
+  cortado_status s = from_cuda(take_room(&ctx->spill, device, (size_t)ctas * BUF_WORDS * 4));  // 14.7 MiB on 148 SMs
+  if (s == CORTADO_OK) s = ensure_flags(ctx, 1024, 0);
   cudaDeviceSynchronize();
   if (s != CORTADO_OK) { cortado_destroy(ctx); return s; }
   *out = ctx;
@@ -1648,9 +1833,10 @@ cortado_status cortado_create(cortado_ctx** out, int device) {
 void cortado_destroy(cortado_ctx* ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
-  cudaDeviceSynchronize();
+  const bool idle = cudaDeviceSynchronize() == cudaSuccess;
   cudaFree(ctx->flags);
   cudaFree(ctx->words);
+  give_room(ctx->spill, idle);
   cudaFree(ctx->d_items);
   cudaFreeHost(ctx->h_items);
   cudaFreeHost(ctx->h_range);
@@ -2079,23 +2265,6 @@ struct NoallocDev {
   int grid = 0;
 };
 
-// The calling thread's current CUDA context (driver entry point, as for the
-// tensor-map encoder), or null when it cannot be queried.
-static CUcontext current_context() {
-  using Fn = CUresult (*)(CUcontext*);
-  static Fn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<Fn>(p);
-  });
-  CUcontext c = nullptr;
-  if (!fn || fn(&c) != CUDA_SUCCESS) return nullptr;
-  return c;
-}
 static NoallocDev g_noalloc_dev[64];
 static std::mutex g_noalloc_mu;
 

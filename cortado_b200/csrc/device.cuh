@@ -63,6 +63,7 @@ struct Sync {
   unsigned int* epoch;        // 0..65535, tags this launch's lookback words
   unsigned long long timeout_ns;
   int resolver;               // encoders: the helper CTA resolves lookback prefixes ahead of the flushes
+  uint32_t* spill;            // re-encoders: BUF_WORDS words per CTA for payloads that do not stay in shared memory
 };
 
 // ---------------------------------------------------------------- PTX helpers

@@ -319,23 +319,54 @@ __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (
   return false;
 }
 
-// A raw chunk's payload from words in global memory (out of line: rare).  Two
-// blocks in flight, read-only loads: the words come from L2 or DRAM (128 MiB of
-// random bits: 110 -> 106 us; four blocks: 110).
-__device__ __noinline__ void flush_words(uint8_t* dst, const uint32_t* words, int nw) {
-  store_payload<2>(dst, 4 * nw, [=](int w) -> uint32_t { return w < nw ? __ldg(words + w) : 0u; });
+// A payload from words in global memory (out of line: rare).  INPUT: a raw
+// chunk's floats, read again; two blocks in flight, read-only loads: the words
+// come from L2 or DRAM (store of 128 MiB of random bits: 110 -> 106 us; four
+// blocks: 110).  Else a compressed payload that this CTA has spilled, padded as
+// it was staged.
+template <bool INPUT>
+__device__ __noinline__ void flush_words(uint8_t* dst, const uint32_t* words, int csize) {
+  if (INPUT)
+    store_payload<2>(dst, csize, [=](int w) -> uint32_t { return 4 * w < csize ? __ldg(words + w) : 0u; });
+  else
+    store_payload<2>(dst, csize, [=](int w) -> uint32_t { return __ldcg(words + staged(w)); });
+}
+// A raw chunk that this CTA has spilled (words 16-byte aligned, 16 readable bytes
+// behind them): 16-byte loads, shifted by the alignment of dst.
+__device__ __noinline__ void flush_raw(uint8_t* dst, const uint32_t* words, int csize) {
+  const int tid = threadIdx.x;
+  const uint8_t* bytes = reinterpret_cast<const uint8_t*>(words);
+  const uint4* w4 = reinterpret_cast<const uint4*>(words);
+  const uintptr_t A = reinterpret_cast<uintptr_t>(dst);
+  const uintptr_t a0 = (A + 15) & ~uintptr_t(15);
+  const uintptr_t a1 = max((A + csize) & ~uintptr_t(15), a0);
+  const int head = min((int)(a0 - A), csize), nblk = (int)((a1 - a0) >> 4);
+#pragma unroll 2
+  for (int b = tid; b < nblk; b += NT) {
+    uint4 x = __ldcg(w4 + b), y = __ldcg(w4 + b + 1);
+    if (head & 8) x = make_uint4(x.z, x.w, y.x, y.y), y = make_uint4(y.z, y.w, 0u, 0u);
+    if (head & 4) x = make_uint4(x.y, x.z, x.w, y.x), y.x = y.y;
+    const uint32_t r = 8u * (head & 3);
+    *reinterpret_cast<uint4*>(a0 + 16 * (uintptr_t)b) =
+        make_uint4(__funnelshift_r(x.x, x.y, r), __funnelshift_r(x.y, x.z, r), __funnelshift_r(x.z, x.w, r),
+                   __funnelshift_r(x.w, y.x, r));
+  }
+  if (tid < head) dst[tid] = __ldcg(bytes + tid);
+  const int at = head + 16 * nblk + tid;
+  if (at < csize) dst[at] = __ldcg(bytes + at);
 }
 
 // Writes out a pending chunk (p; its output offset in sm.payload_off; both
-// visible after a barrier) from its staging buffer -- or, for a raw chunk, from
-// raw_words, when not null (else its words are staged too) -- and
+// visible after a barrier) from its staging buffer -- or from raw_words, the
+// input's floats, for a raw chunk of the store (FLOATS) -- and
 // its size-table entry; the stream's last chunk also sets the stream size.
+template <bool FLOATS>
 __device__ __forceinline__ void flush_staged(const Ctl& sm, const Pend& p, const uint32_t* st, const uint32_t* st_small,
                                              const uint32_t* raw_words, uint8_t* data_out, uint16_t* table_out,
                                              long long* out_size, long long chunks) {
   const unsigned long long X = sm.payload_off;
-  if (p.raw && raw_words) {
-    flush_words(data_out + X, raw_words, p.nw);
+  if (FLOATS && p.raw) {
+    flush_words<true>(data_out + X, raw_words, p.csize);
   } else {
     if (p.small) st = st_small;
     const uint32_t pad = p.small ? 31 : 5;  // no padding, or staged()

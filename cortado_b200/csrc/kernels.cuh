@@ -110,12 +110,15 @@ struct __align__(16) Ctl {
   uint64_t bar;             // a chunk's loads
   uint64_t bar_src;         // resi_recv: the client chunk
   StageMeta st[2];
-  Pend pend[2];             // encoders: the chunks whose payloads wait to be flushed
+  Pend pend[2];             // encoders: the chunks whose payloads wait to be flushed (re-encoders: [1] a spilled one)
   unsigned long long payload_off;
   unsigned int epoch, is_last;
   unsigned int first;       // the CTA's first place in the queue (all ones: the helper)
-  unsigned int held;        // re-encoders: the next payload waits for room
+  unsigned int held;        // re-encoders: bit 0: the next payload waits for room; bit 1: pend[1] is to be flushed
   unsigned int src_side;    // resi_recv: this chunk's client floats are behind the next payload
+  unsigned int zeros;       // re-encoders: chunks of zeros whose 2-byte payloads wait for their offsets
+  uint32_t zero_c[32];      //   (chunk and item of each; one warp's alone)
+  int zero_item[32];
 };
 static_assert(sizeof(Ctl) <= CTL_BYTES, "control block");
 
