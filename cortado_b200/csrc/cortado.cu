@@ -44,9 +44,10 @@ __device__ __forceinline__ Ctl& ctl_block() {
   return *reinterpret_cast<Ctl*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 }
 
-// The thread that issues every TMA load and store of a CTA (warp 3, lane 0):
-// bulk-store completion is tracked per thread, so the thread that reuses a
-// buffer after a TMA store must be the one that issued the store.
+// The thread that issues a decoder's TMA loads and stores (warp 3, lane 0):
+// bulk-store completion is tracked per thread, so the thread that loads over a
+// buffer after a TMA store must be the one that issued the store.  (The encoders
+// have no TMA stores; lane 0 of their warp 1 issues the loads.)
 constexpr int TMA_TID = 96;
 
 // Start of every CTA: takes its place in the launch's queue, reads the lookback
@@ -234,8 +235,8 @@ __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* m) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(m) : "memory");
 }
 
-// ---- prefetchers (warp 3): resolve queue index g and start its loads into
-// stage t.  Every TMA is issued by lane 0 (TMA_TID).
+// ---- the store's prefetch (its loader warp): finds the chunk of queue index g
+// and starts its load into buffer t; lane 0 issues it.
 struct WalkState {
   int item;                 // item of the last prefetched index (-1: none)
 };
@@ -281,12 +282,14 @@ __device__ __forceinline__ void prefetch_floats(Ctl& sm, int t, long long g, con
 }
 
 // ---- the three pipelined loops.  Each CTA dequeues chunk indices from the
-// launch's queue; warp 3 resolves an index and starts its loads.  Decoders
-// take their indices one iteration ahead and load the next chunk while the
-// current one is decoded; encoders take an index when they start the chunk.
+// launch's queue; one warp (warp 1 of the encoders, warp 3 of the decoders)
+// finds the chunk and starts its loads.  Decoders take their indices one
+// iteration ahead, re-encoders once the present chunk has been expanded, the
+// store once its planes are written; each loads the next chunk as soon as a
+// buffer has room for it.
 //
 // Encoders publish a chunk's compressed size as soon as it is known and write
-// its payload one iteration later (flush_chunk): by then every earlier chunk
+// its payload one iteration later (write_pending): by then every earlier chunk
 // has published too, and the resolver CTA has usually turned the chunk's own
 // lookback word into an inclusive prefix, so no CTA waits on its
 // predecessors while it holds the SM.
@@ -869,12 +872,11 @@ __device__ __noinline__ void zero_chunk(Ctl& sm, const Src src, const StageMeta&
 // compress stores its requantized words, which are rebuilt from the planes
 // (planes_to_words) and always spilled.
 // (Decoding in place in one buffer and staging in the other took 11 barriers a
-// chunk; this takes 7.  256 MiB: init_send 462 -> 320 us and resi_send 468 ->
-// 340 us on sinusoids with noise, 552 -> 414 and 516 -> 387 us on dense data,
-// 269 -> 256 and 282 -> 277 us on nearly all zero bins.  Instruction fetch was
-// then the largest stall; the loops of planes_to_words, rze_decode and
-// encode_chunk that are not unrolled brought init_send to 294, 373 and 245 us,
-// resi_send to 320, 370 and 266 us.)
+// chunk; this takes 7.  Instruction fetch is then the largest stall beside them,
+// hence the loops of planes_to_words, rze_decode and encode_chunk that are not
+// unrolled.  128 MiB, init_send and resi_send: sinusoids with noise 252 -> 137 us
+// and 256 -> 141, dense data 342 -> 245 and 351 -> 242, nearly all zero bins 159 ->
+// 148 and 103 -> 91.)
 // APPLY: the fused send-and-apply forms (items with a client's floats); the
 // plain forms are compiled without that code.
 template <int OP, bool APPLY, class Src>

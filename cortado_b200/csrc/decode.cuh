@@ -2,16 +2,15 @@
 // RZE_1, BIT_4 and DIFFMS of one 16 KiB chunk in a 128-thread CTA, 32 words
 // per thread (the layouts of device.cuh).
 //
-// What bounds them: the integer pipe (busy 55-65% of the cycles) and the
-// barriers between the dependent phases of a chunk, not DRAM (14-20%).  So the
+// What bounds them: the integer pipe (busy 40-50% of the cycles) and the
+// barriers between the dependent phases of a chunk, not DRAM (17-38%).  So the
 // bitmap levels are rebuilt with byte permutes instead of chains of dependent
 // loads, every warp derives the small levels itself, and the payload and the
 // planes have a buffer each: two barriers fewer than with one for both, and
 // the next payload arrives while this one's planes are turned into floats.
-// Instructions per chunk 5,048 -> 4,472 on a field of nearly all zero bins.
-// On 256 MiB: init_recv 132 -> 121 us (zero bins), 187 -> 147 (sinusoids with
-// noise, 6% of the size), 200 -> 167 (25%); storage decode 200 -> 160 at 31%;
-// resi_recv 202 -> 162, 265 -> 200, 286 -> 222.
+// Instructions per chunk 5,048 -> 3,900 on a field of nearly all zero bins.
+// 128 MiB: init_recv 97 -> 65 us (sinusoids with noise, 14% of the size), 121 ->
+// 84 (dense, 66%); storage decode 101 -> 69 at 30%; resi_recv 136 -> 85.
 // Two threads per 32-word group (16 words each, up to 48 warps per SM instead
 // of 24) measured slower (148, 174, 188 us for init_recv): the added warps
 // repeat the scans and bitmap levels, and the pipe was the limit already.

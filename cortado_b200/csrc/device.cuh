@@ -252,11 +252,11 @@ __device__ __forceinline__ uint32_t iq_mixed(uint32_t b, const FastQ& f, const Q
 // recursive block-swap transpose (H. S. Warren, Hacker's Delight, 2nd ed.,
 // sec. 7-3); the 16- and 8-bit stages are byte permutes.  The transform is an
 // involution, so the decoder applies the same function.
+
 // (y & m) | (x & ~m) in one instruction.  Two shifts and two selects per pair
 // of rows instead of two shifts and three exclusive-ors: every kernel ran 2-6%
-// faster (256 MiB: store 168 -> 158 us on zero bins, init_send 495 -> 476 us on
-// sinusoids with noise); written as plain C the compiler made more than that
-// of it, and both were slower.
+// faster; written as plain C the compiler made more than that of it, and it was
+// slower than the exclusive-ors.
 __device__ __forceinline__ uint32_t bit_select(uint32_t x, uint32_t y, uint32_t m) {
   uint32_t r;
   asm("lop3.b32 %0, %1, %2, %3, 0xd8;" : "=r"(r) : "r"(x), "r"(y), "r"(m));
@@ -286,11 +286,6 @@ __device__ __forceinline__ void transpose_blocks(uint32_t (&a)[N]) {
   swap_stage<2>(a, 0x33333333u);
   swap_stage<1>(a, 0x55555555u);
 }
-// Full groups are transposed one half of the planes at a time: words k and
-// k + 16 share a register (their high halves for planes 0..15, their low halves
-// for planes 16..31), and the stages run on 16 registers.  The pass for planes
-// that are zero in the whole warp is left out, and both passes are the same
-// code.
 
 // ---------------------------------------------------------------- byte masks
 // 4-bit mask of the non-zero bytes of x (bit b <-> byte b).

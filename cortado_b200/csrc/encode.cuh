@@ -3,12 +3,12 @@
 // raw fallback, and the staging of the payload until its output offset is
 // known.
 //
-// What bounds it: the integer pipe (47-54% busy) and the barriers between a
+// What bounds it: the integer pipe (52-57% busy) and the barriers between a
 // chunk's phases (half the stalls), not DRAM.  Hence:
 //   * words below 2^16 (nearly all differences of neighbours) are transposed in
 //     16 registers instead of 32;
 //   * the zero-byte bitmap comes from byte dot products (36 instructions for
-//     eight words, 56 with shifts and multiplies: 175 against 185 us below);
+//     eight words; 56 with shifts and multiplies, and the store took 5% longer);
 //   * the payload is packed from registers into full words (15 instructions a
 //     word) instead of byte by byte, over the planes, whose buffer no thread
 //     reads any more; the other buffer is free for the next chunk's input;
@@ -16,8 +16,8 @@
 //     to being stored raw;
 //   * few bytes are written one by one, behind the planes: the packing's fixed
 //     cost is higher than theirs.
-// Store of 256 MiB: 297 -> 175 us (sinusoids with noise, 31% of the size), 347
-// -> 230 (60%), 167 -> 158 (nearly all zero bins).
+// Store of 128 MiB: 151 -> 80 us (sinusoids with noise, 30% of the size), 174 ->
+// 114 (dense, 82%), 94 -> 85 (nearly all zero bins).
 #pragma once
 #include "decode.cuh"
 
@@ -98,8 +98,12 @@ struct Packer {
 // Three hooks run on every thread: planes_written() before the barrier after
 // which the planes are read, planes_ready() after it, and planes_read(n) after
 // the next one, with a bound n of the payload's bytes.
-// KEEP: the plane words stay in registers (st is Y); else they are read again for the packing, eight at a time in a loop, which keeps
-// the re-encoders' code short.  ZEROS: the words may all be zero (else the caller
+// Full groups are transposed one half of the planes at a time: words k and k + 16
+// share a register (their high halves for planes 0..15, their low halves for
+// planes 16..31), and the stages run on 16 registers.  The pass for planes that
+// are zero in the whole warp is left out, and both passes are the same code.
+// KEEP: the plane words stay in registers (st is Y); else they are read again for
+// the packing, eight at a time in a loop, which keeps the re-encoders' code short.  ZEROS: the words may all be zero (else the caller
 // has seen to such chunks).
 template <bool KEEP, bool ZEROS, typename Written, typename Ready, typename Read>
 __device__ __forceinline__ bool encode_chunk(Ctl& sm, const Sync& sy, uint32_t (&v)[32], uint32_t prev0, uint32_t* Y,

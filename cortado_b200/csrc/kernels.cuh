@@ -239,6 +239,7 @@ __device__ __noinline__ void compact_planes(uint32_t* Y, int nw) {
 // transposes them back, undoes the zig-zag and the differences (in-thread
 // prefix sum plus a block scan of the group totals), and returns the group's
 // words in v[32] and the word before them in `before` (0 for the first group).
+// The planes are taken a half at a time, as encode_chunk writes them.
 // (Words behind a partial chunk's end repeat its last one.)  Ends with a
 // barrier (the scan's), after which the plane buffer may be reused.  SHORT:
 // loops are not unrolled (the re-encoders, whose code is long).
