@@ -517,10 +517,34 @@ __device__ __forceinline__ void park_stream(Ctl& sm, int t, const Src& src, cons
 // has not published their offset yet: at most eight loads per lane.
 constexpr int OWN_SUM = 256;
 
+// The offset of a payload that the scanner had not published when the chunk was
+// taken (one warp).
+__device__ __forceinline__ unsigned long long open_offset(const OpArgs& A, long long c, unsigned int epoch) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long off = 0;
+  if (c < OWN_SUM) {
+    // (the scanner is still starting: a small launch would wait for it)
+    unsigned int sum = 0;
+    const uint16_t* table = reinterpret_cast<const uint16_t*>(A.in + HDR);
+    for (int i = lane; i < (int)c; i += 32) sum += table[i];
+    off = __reduce_add_sync(0xffffffffu, sum);
+  } else {
+    if (lane == 0) off = wait_offset(A.sy, epoch, c);
+    off = __shfl_sync(0xffffffffu, off, 0);
+  }
+  return off;
+}
+__device__ __noinline__ unsigned long long open_offset_far(const OpArgs& A, long long c, unsigned int epoch) {
+  return open_offset(A, c, epoch);
+}
+
 // Second part, once the place at byte `at` (a multiple of 16) of P is free: the
 // payload's 16-byte-aligned span with one bulk copy, the ragged tail by the
-// lanes.
-template <class Src>
+// lanes.  FAR: the rare wait for an offset is out of line.  The re-encoders hold
+// five copies of this, and instruction fetch is their largest stall (128 MiB:
+// init_send 152 -> 148 us on nearly all zero bins, init_send_apply 156 -> 152 on
+// sinusoids with noise); resi_recv ran 2% slower with it.
+template <bool FAR, class Src>
 __device__ __forceinline__ void issue_stream(Ctl& sm, int t, const Src& src, uint8_t* P, int at) {
   const int lane = threadIdx.x & 31;
   StageMeta& m = sm.st[t];
@@ -538,15 +562,8 @@ __device__ __forceinline__ void issue_stream(Ctl& sm, int t, const Src& src, uin
   unsigned long long off = m.off;
   if ((off >> 48) == sm.epoch && (off & LB_INC)) {
     off &= LB_VAL;
-  } else if (m.c < OWN_SUM) {
-    // (the scanner is still starting: a small launch would wait for it)
-    unsigned int sum = 0;
-    const uint16_t* table = reinterpret_cast<const uint16_t*>(A.in + HDR);
-    for (int i = lane; i < (int)m.c; i += 32) sum += table[i];
-    off = __reduce_add_sync(0xffffffffu, sum);
   } else {
-    if (lane == 0) off = wait_offset(A.sy, sm.epoch, m.c);
-    off = __shfl_sync(0xffffffffu, off, 0);
+    off = FAR ? open_offset_far(A, m.c, sm.epoch) : open_offset(A, m.c, sm.epoch);
   }
   const int cs = m.csize;
   __syncwarp();  // (lane 0 rewrites it below)
@@ -901,7 +918,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
     if (feeder) park_stream(sm, t, src, ah);
   };
   auto issue = [&](int t) {  // (feeder)
-    issue_stream(sm, t, src, reinterpret_cast<uint8_t*>(R), ROOM - room_in(min(sm.st[t].csize, CS)));
+    issue_stream<true>(sm, t, src, reinterpret_cast<uint8_t*>(R), ROOM - room_in(min(sm.st[t].csize, CS)));
   };
   resolve(0, sm.first);
   park(0);
@@ -913,7 +930,7 @@ __device__ __forceinline__ void reencode_loop(Ctl& sm, const Src& src, const Syn
     const OpArgs& A = src.args(m.item);
     const ChunkKind kind = rze_decode<true>(sm, A.sy, m, R, Y, NoHook{});
     const unsigned int g = take();
-    if (m.bad >= 2) {  // unusable stream header (batched): nothing to write
+    if (Src::batched && m.bad >= 2) {  // unusable stream header (batched): nothing to write
       resolve(s ^ 1, g);
       park(s ^ 1);
       flush_now(sm, src, R, spill);
@@ -1068,7 +1085,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     resolve_stream<OP>(sm, 0, sm.first, src, ws, ah);
     if (lane == 0) pending = next_place(sy);
     park_stream(sm, 0, src, ah);
-    issue_stream(sm, 0, src, reinterpret_cast<uint8_t*>(P), 0);
+    issue_stream<OP != OP_RAPPLY>(sm, 0, src, reinterpret_cast<uint8_t*>(P), 0);
   }
   uint32_t phase = 0;  // bit 0: payload; bit 1: client chunk
   for (int s = 0;; s ^= 1) {
@@ -1103,7 +1120,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
         q_free();
         park_stream(sm, s ^ 1, src, ah);
         asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
-        issue_stream(sm, s ^ 1, src, reinterpret_cast<uint8_t*>(Q), 0);
+        issue_stream<OP != OP_RAPPLY>(sm, s ^ 1, src, reinterpret_cast<uint8_t*>(Q), 0);
       } else {
         asm volatile("bar.arrive 1, %0;" ::"n"(NT) : "memory");
       }
@@ -1123,7 +1140,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
     const ChunkKind kind = rze_decode<OP == OP_RAPPLY>(sm, A.sy, m, P, Q, q_free);
     if (feeder) {
       park_stream(sm, s ^ 1, src, ah);
-      issue_stream(sm, s ^ 1, src, reinterpret_cast<uint8_t*>(P), 0);
+      issue_stream<OP != OP_RAPPLY>(sm, s ^ 1, src, reinterpret_cast<uint8_t*>(P), 0);
       if (OP == OP_RAPPLY && lane == 0) {
         // When the next payload fills at most the first KiB of P, this chunk's
         // client floats are loaded behind it (1024-byte aligned) now.
@@ -1137,7 +1154,7 @@ __device__ __forceinline__ void decode_loop(Ctl& sm, const Src& src, const Sync&
         }
       }
     }
-    if (m.bad >= 2) {  // unusable stream header (batched): nothing to write
+    if (Src::batched && m.bad >= 2) {  // unusable stream header (batched): nothing to write
       __syncthreads();  // every warp has read m.bad: the feeder may take this slot again at once
       continue;
     }
