@@ -2,13 +2,13 @@
 // RZE_1, BIT_4 and DIFFMS of one 16 KiB chunk in a 128-thread CTA, 32 words
 // per thread (the layouts of device.cuh).
 //
-// What bounds them: the integer pipe (busy 40-50% of the cycles) and the
+// What bounds them: the integer pipe (busy 39-44% of the cycles) and the
 // barriers between the dependent phases of a chunk, not DRAM (17-38%).  So the
 // bitmap levels are rebuilt with byte permutes instead of chains of dependent
 // loads, every warp derives the small levels itself, and the payload and the
 // planes have a buffer each: two barriers fewer than with one for both, and
 // the next payload arrives while this one's planes are turned into floats.
-// Instructions per chunk 5,048 -> 3,900 on a field of nearly all zero bins.
+// Instructions per chunk 5,048 -> 3,831 on a field of nearly all zero bins.
 // 128 MiB: init_recv 97 -> 65 us (sinusoids with noise, 14% of the size), 121 ->
 // 84 (dense, 66%); storage decode 101 -> 69 at 30%; resi_recv 136 -> 85.
 // Two threads per 32-word group (16 words each, up to 48 warps per SM instead

@@ -3,7 +3,7 @@
 // raw fallback, and the staging of the payload until its output offset is
 // known.
 //
-// What bounds it: the integer pipe (52-57% busy) and the barriers between a
+// What bounds it: the integer pipe (48-51% busy) and the barriers between a
 // chunk's phases (half the stalls), not DRAM.  Hence:
 //   * words below 2^16 (nearly all differences of neighbours) are transposed in
 //     16 registers instead of 32;

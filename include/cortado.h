@@ -62,7 +62,9 @@ int64_t cortado_max_stream_bytes(int64_t n_bytes);
  * (reference include/d_server_encode.h:150-158). */
 cortado_status cortado_eb_exponent(float eb_abs, int* biased_exponent);
 
-/* Context: scratch (lookback words, chunk queue, status word) on `device`. */
+/* Context: scratch (lookback words, chunk queue, status word, and room for one
+ * payload per CTA of the send kernels, 14.7 MiB on a B200) on `device`.  The room of
+ * up to four destroyed contexts is kept for the next ones. */
 cortado_status cortado_create(cortado_ctx** ctx, int device);
 void cortado_destroy(cortado_ctx* ctx);
 /* Upper bound of every device-side wait (default 2 s). */
